@@ -40,6 +40,7 @@
 
 #include "../../include/pgx.h"
 #include "pgx_device.cuh"
+#include "pgx_flow.cuh"
 #include "pgx_internal.h"
 #include "pgx_umma.cuh"
 #include "pgx_systems.cuh"
@@ -262,21 +263,6 @@ static SpmvPlan spmv_plan(int rows, const int* rp) {
 // merge-path threads (kMergeItems items each) for a rows x nnz matrix
 static int merge_threads(long long rows, long long nnz) { return (int)((rows + nnz + kMergeItems - 1) / kMergeItems); }
 
-// Lanes per row of the per-subdomain solve: about PGX_PIPE_NNZ_PER_LANE nonzeros
-// per lane, so that a row's operand loads are issued at once (kUnroll deep)
-// and a level of a few dozen rows needs one sweep of the CTA's groups.  The
-// choice depends on the factor alone, so every slot and lane count of a
-// handle sums each row in the same order.
-#ifndef PGX_PIPE_NNZ_PER_LANE
-#define PGX_PIPE_NNZ_PER_LANE 4
-#endif
-static int pipe_lanes(long long nnz, long long rows) {
-  const double avg = rows > 0 ? (double)nnz / (double)rows : 0.0;
-  int S = 2;
-  while (S < 16 && avg > (double)PGX_PIPE_NNZ_PER_LANE * S) S *= 2;
-  return S;
-}
-
 // -------------------------------------------------------- device memory
 struct Arena {
   std::vector<void*> ptrs;
@@ -358,13 +344,11 @@ struct DTri {
   unsigned long long* ticket = nullptr;
   // segmented schedule (trsv_seg_kernel); seg == false uses trsv_kernel
   bool seg = false;
-  bool comp = false;  // one CTA per subdomain (trsv_pipe_kernel)
+  bool comp = false;  // one CTA per subdomain (trsv_flow_kernel)
   int nseg = 0, ncomp = 1;
-  int *comp_ch0 = nullptr, *cmeta = nullptr, *far_col = nullptr;  // one-CTA-per-subdomain schedule
-  T* dslot = nullptr;   // upper pass: inverse diagonal in slot order
-  int* uslot = nullptr; // lower pass: upper-pass slot of each row, in slot order
-  int nslots = 0;       // length of the slot arrays (padded row list)
-  int nslots_up = 0;    // lower pass: length of the yslot vector it fills (the upper layout's nslots)
+  FlowArgs flow{};         // one-CTA-per-subdomain schedule
+  bool flow_long = false;  // laid out for the longer ring
+  long long flow_tasks = 0, flow_far = 0;
   long long nnz_total = 0;  // nonzeros of the factor (without padding)
   int *seg_row0 = nullptr, *seg_rp0 = nullptr, *seg_nnz0 = nullptr, *seg_lv0 = nullptr, *seg_nlvb = nullptr,
       *lvb = nullptr;
@@ -552,199 +536,65 @@ static int upload_tri_seg(Arena& ar, const HostCsr& h, bool upper, const std::ve
   return PGX_SUCCESS;
 }
 
-// Chunked per-subdomain schedule for trsv_pipe_kernel: each subdomain's
-// rows in level-set order, cut into chunks that fit the kernel's staging
-// buffers, subdomain after subdomain.  A dependency is encoded as the
-// negative ring slot -(q % ring + 1) when its schedule position q is close
-// enough that no row of the consumer's level can have overwritten the slot
-// (end of the consumer's level - q < ring); otherwise as the row index, read
-// back from global memory.  Returns PGX_ERROR_INVALID_PARAM (and builds
-// nothing) when the factor couples two subdomains.
-template <typename T, typename CC>
-static int upload_tri_sub(Arena& ar, const HostCsr& h, bool upper, const std::vector<int>& dom, DTri<T>& d,
-                          cudaStream_t s, const std::vector<double>* dinv, std::vector<int>* slot_of_row,
-                          const std::vector<int>* upper_slot_of_row);
-template <typename T>
-static int upload_tri_comp(Arena& ar, const HostCsr& h, bool upper, const std::vector<int>& dom, DTri<T>& d,
+// The per-subdomain schedule of trsv_flow_kernel for R right-hand sides.
+// Returns PGX_ERROR_INVALID_PARAM (and builds nothing) when the factor does
+// not suit the kernel (it couples two subdomains, or a row is too long).
+template <typename T, int R>
+static int upload_tri_flow(Arena& ar, const HostCsr& h, bool upper, const std::vector<int>& dom, DTri<T>& d,
                            cudaStream_t s, const std::vector<double>* dinv, std::vector<int>* slot_of_row,
                            const std::vector<int>* upper_slot_of_row) {
-  return upload_tri_sub<T, PipeCfg<T, 1>>(ar, h, upper, dom, d, s, dinv, slot_of_row, upper_slot_of_row);
-}
-
-// The layout for a per-subdomain kernel whose shared-memory sizes are CC's.
-template <typename T, typename CC>
-static int upload_tri_sub(Arena& ar, const HostCsr& h, bool upper, const std::vector<int>& dom, DTri<T>& d,
-                          cudaStream_t s, const std::vector<double>* dinv, std::vector<int>* slot_of_row,
-                          const std::vector<int>* upper_slot_of_row) {
+  using C = FlowCfg<T, R>;
   const int n = h.rows;
-  std::vector<int> lptr, order, lev;
-  PGX_TRY(build_levels(upper, n, h.rp.data(), h.cj.data(), lptr, order, &lev));
   std::vector<int> cuts = dom;
   bool ok = cuts.size() >= 2 && cuts.front() == 0 && cuts.back() == n;
   for (size_t c = 0; ok && c + 1 < cuts.size(); c++) ok = cuts[c] <= cuts[c + 1];
   if (!ok) cuts = {0, n};
-  const int ncomp = (int)cuts.size() - 1;
-  std::vector<int> comp_of(n);
-  for (int c = 0; c < ncomp; c++)
-    for (int r = cuts[c]; r < cuts[c + 1]; r++) comp_of[r] = c;
-  for (int r = 0; r < n; r++)
-    for (int k = h.rp[r]; k < h.rp[r + 1]; k++)
-      if (comp_of[h.cj[k]] != comp_of[r]) return PGX_ERROR_INVALID_PARAM;
-  for (int r = 0; r < n; r++)
-    if (h.rp[r + 1] - h.rp[r] > CC::nnz - 4) return PGX_ERROR_INVALID_PARAM;
-  // positions inside each subdomain, in level order
-  std::vector<std::vector<int>> sched(ncomp);
-  for (int p = 0; p < n; p++) sched[comp_of[order[p]]].push_back(order[p]);
-  std::vector<int> posc(n), lvl_end(n);
-  for (int c = 0; c < ncomp; c++) {
-    auto& sc = sched[c];
-    for (size_t p = 0; p < sc.size(); p++) posc[sc[p]] = (int)p;
-    // end position (exclusive) of each row's level
-    size_t a = 0;
-    while (a < sc.size()) {
-      size_t e = a;
-      while (e < sc.size() && lev[sc[e]] == lev[sc[a]]) e++;
-      for (size_t p = a; p < e; p++) lvl_end[sc[p]] = (int)e;
-      a = e;
+  FlowPack<T> pk;
+  auto val = [&](int k) { return hval<T>(h.va.data(), (size_t)k); };
+  auto diag = [&](int i) { return hval<T>(dinv->data(), (size_t)i); };
+  const bool fits = flow_pack<T, C>(n, h.rp.data(), h.cj.data(), val, upper, cuts, &diag, upper_slot_of_row, pk);
+  // Operands that left the ring are read back from global memory.  When they
+  // are more than a hundredth of the entries, a ring twice as long with fewer
+  // warps is the better trade (FP64, four lanes: 128^3, 30% of the entries
+  // far, 19.7 ms against 11.4 ms with the longer ring; 64^3, 0.1% far, 1.00
+  // ms against 1.14 ms).
+  d.flow_long = false;
+  if constexpr (C::has_long) {
+    if (!fits || pk.nfar * 100 > h.nnz()) {
+      FlowPack<T> lk;
+      if (flow_pack<T, FlowCfg<T, R, true>>(n, h.rp.data(), h.cj.data(), val, upper, cuts, &diag, upper_slot_of_row,
+                                            lk) &&
+          (!fits || 2 * lk.nfar < pk.nfar)) {
+        d.flow_long = true;
+        std::swap(pk, lk);
+      }
     }
   }
-  auto pad4 = [](std::vector<int>& v, int fill) {
-    while (v.size() % 4) v.push_back(fill);
-  };
-  const int ROWCAP = CC::rows - 4, NNZCAP = CC::nnz - 4;
-  // near operands stay in the shared ring until the consumer reads them:
-  // within `ring` positions of the end of the consumer's level
-  auto is_near = [&](int r, int qj) { return lvl_end[r] - qj < CC::ring; };
-  std::vector<int> nfar(n, 0);
-  for (int r = 0; r < n; r++)
-    for (int k = h.rp[r]; k < h.rp[r + 1]; k++)
-      if (!is_near(r, posc[h.cj[k]])) nfar[r]++;
-  for (int r = 0; r < n; r++)
-    if (nfar[r] > CC::far) return PGX_ERROR_INVALID_PARAM;
-  std::vector<int> ord, rp, cj, lvb, meta, comp_ch0(1, 0), far_col;
-  std::vector<T> va;
-  auto push_meta = [&](int pos0) {
-    meta.insert(meta.end(), {(int)ord.size(), (int)rp.size(), (int)cj.size(), (int)lvb.size(), pos0,
-                             (int)far_col.size(), 0, 0});
-  };
-  for (int c = 0; c < ncomp; c++) {
-    const auto& sc = sched[c];
-    size_t p = 0;
-    // starts of the previous chunk and of the one before it: a chunk's far
-    // operands are gathered while the chunk two before it is solved, so they
-    // must lie before that chunk's start
-    int prev_start = 0, prev2_start = 0, chunk_in_comp = 0;
-    while (p < sc.size()) {
-      // one chunk: consecutive positions within the row, nonzero and far caps
-      size_t e = p;
-      long long nz = 0;
-      int nf = 0;
-      while (e < sc.size() && (int)(e - p) < ROWCAP) {
-        const int rn = h.rp[sc[e] + 1] - h.rp[sc[e]];
-        if (nz + rn > NNZCAP || nf + nfar[sc[e]] > CC::far) break;
-        nz += rn;
-        nf += nfar[sc[e]];
-        e++;
-      }
-      push_meta((int)p);
-      const int far_base = CC::ring + (chunk_in_comp % 3) * CC::far;
-      const int far0 = (int)far_col.size();
-      rp.push_back(0);
-      int acc = 0;
-      for (size_t q = p; q < e; q++) {
-        const int r = sc[q];
-        ord.push_back(r);
-        for (int k = h.rp[r]; k < h.rp[r + 1]; k++) {
-          const int j = h.cj[k];
-          const int qj = posc[j];
-          if (is_near(r, qj)) {
-            cj.push_back(-((qj & (CC::ring - 1)) + 1));
-          } else {
-            // far: gathered while the chunk two before is solved, so it
-            // must have been published before that chunk began
-            if (qj >= prev2_start) return PGX_ERROR_INVALID_PARAM;
-            cj.push_back(-(far_base + ((int)far_col.size() - far0) + 1));
-            far_col.push_back(j);
-          }
-          va.push_back(hval<T>(h.va.data(), k));
-        }
-        acc += h.rp[r + 1] - h.rp[r];
-        rp.push_back(acc);
-      }
-      pad4(ord, -1);
-      pad4(rp, acc);
-      pad4(far_col, -1);
-      while (cj.size() % 4) {
-        cj.push_back(0);
-        va.push_back(T(0.0));
-      }
-      lvb.push_back(0);
-      for (size_t q = p + 1; q < e; q++)
-        if (lev[sc[q]] != lev[sc[q - 1]]) lvb.push_back((int)(q - p));
-      lvb.push_back((int)(e - p));
-      pad4(lvb, (int)(e - p));
-      prev2_start = prev_start;
-      prev_start = (int)p;
-      chunk_in_comp++;
-      p = e;
-    }
-    comp_ch0.push_back((int)meta.size() / 8);
-  }
-  push_meta(0);  // closes the last chunk
-  for (int c : cj)
-    if (c >= 0 || -c - 1 >= CC::ring + 3 * CC::far)
-      if (c != 0) return fail(PGX_ERROR_INVALID_PARAM, "per-subdomain layout: operand index out of range");
-  // every chunk is staged by bulk copies: each range starts on a 16-byte
-  // boundary, spans a multiple of 16 bytes and fits its staging buffer
-  for (size_t ch = 0; ch + 1 < meta.size() / 8; ch++) {
-    const int* m = &meta[ch * 8];
-    const int* e = &meta[(ch + 1) * 8];
-    const int nr = e[0] - m[0], np = e[1] - m[1], nz = e[2] - m[2], nv = e[3] - m[3], nf = e[5] - m[5];
-    const bool aligned = (m[0] | m[1] | m[2] | m[3] | m[5] | nr | np | nz | nv | nf) % 4 == 0;
-    const bool fits = nr > 0 && nr <= CC::rows && np <= CC::rows + 4 && nv <= CC::rows + 4 && nz <= CC::nnz &&
-                      nf <= CC::far && np > 0 && nv > 0 && nz >= 0 && nf >= 0;
-    if (!aligned || !fits)
-      return fail(PGX_ERROR_INVALID_PARAM, "per-subdomain layout: chunk %zu breaks the staging rules", ch);
-  }
-  // slot of every row in the flat row list; the upper pass's slots index its
-  // dinv and the y the lower pass leaves behind
-  std::vector<int> slot(n, -1);
-  for (size_t i = 0; i < ord.size(); i++)
-    if (ord[i] >= 0) slot[ord[i]] = (int)i;
-  std::vector<T> dsl;
-  std::vector<int> usl;
-  if (upper) {
-    dsl.assign(ord.size(), T(0.0));
-    for (size_t i = 0; i < ord.size(); i++)
-      if (ord[i] >= 0) dsl[i] = hval<T>(dinv->data(), ord[i]);
-  } else {
-    usl.assign(ord.size(), 0);
-    for (size_t i = 0; i < ord.size(); i++)
-      if (ord[i] >= 0) usl[i] = (*upper_slot_of_row)[ord[i]];
-  }
-  if (slot_of_row) *slot_of_row = slot;
+  if (!fits && !d.flow_long) return PGX_ERROR_INVALID_PARAM;
   d.n = n;
   d.comp = true;
   d.seg = false;
-  d.ncomp = ncomp;
-  d.nslots = (int)ord.size();
-  d.nlevels = (int)lptr.size() - 1;
-  d.nseg = (int)meta.size() / 8 - 1;
+  d.ncomp = pk.ncomp;
+  d.nlevels = pk.nlevels;
+  d.nseg = (int)pk.chunk.size() / 4;
   d.nnz_total = h.nnz();
-  d.S = pipe_lanes(h.nnz(), n);
-  d.nblocks = ncomp;
-  PGX_TRY(ar.upload(&d.ord, ord.data(), ord.size(), s));
-  PGX_TRY(ar.upload(&d.rp, rp.data(), rp.size(), s));
-  PGX_TRY(ar.upload(&d.cj, cj.data(), cj.size(), s));
-  PGX_TRY(ar.upload(&d.va, va.data(), va.size(), s));
-  PGX_TRY(ar.upload(&d.lvb, lvb.data(), lvb.size(), s));
-  PGX_TRY(ar.upload(&d.cmeta, meta.data(), meta.size(), s));
-  PGX_TRY(ar.upload(&d.comp_ch0, comp_ch0.data(), comp_ch0.size(), s));
-  PGX_TRY(ar.upload(&d.far_col, far_col.data(), far_col.size(), s));
-  if (upper)
-    PGX_TRY(ar.upload(&d.dslot, dsl.data(), dsl.size(), s));
-  else
-    PGX_TRY(ar.upload(&d.uslot, usl.data(), usl.size(), s));
+  d.nblocks = pk.ncomp;
+  d.flow_tasks = pk.ntasks;
+  d.flow_far = pk.nfar;
+  int *chunk = nullptr, *first = nullptr, *comp0 = nullptr;
+  unsigned char* blob = nullptr;
+  PGX_TRY(ar.upload(&chunk, pk.chunk.data(), pk.chunk.size(), s));
+  PGX_TRY(ar.upload(&comp0, pk.comp_chunk0.data(), pk.comp_chunk0.size(), s));
+  PGX_TRY(ar.upload(&first, pk.first.data(), pk.first.size(), s));
+  PGX_TRY(ar.alloc(&blob, pk.blob.size()));
+  PGX_CUDA(cudaMemcpyAsync(blob, pk.blob.data(), pk.blob.size(), cudaMemcpyHostToDevice, s));
+  PGX_CUDA(cudaStreamSynchronize(s));
+  d.flow.n = n;
+  d.flow.chunk = (const int4*)chunk;
+  d.flow.comp_chunk0 = comp0;
+  d.flow.first = (const int2*)first;
+  d.flow.blob = blob;
+  if (slot_of_row) slot_of_row->swap(pk.slot_of_row);
   return PGX_SUCCESS;
 }
 
@@ -778,8 +628,8 @@ static std::string describe_tri(const char* what, const DTri<T>& t) {
   if (t.n == 0) {
     snprintf(buf, sizeof(buf), "  %s: empty\n", what);
   } else if (t.comp) {
-    snprintf(buf, sizeof(buf), "  %s: per-subdomain pipeline, %d CTAs, %d lanes per row, %d dependency levels, %d chunks, %lld nonzeros\n",
-             what, t.ncomp, t.S, t.nlevels, t.nseg, t.nnz_total);
+    snprintf(buf, sizeof(buf), "  %s: per-subdomain dataflow, %d CTAs, %d dependency levels, %lld tasks, %d chunks, %lld nonzeros (%lld far)\n",
+             what, t.ncomp, t.nlevels, t.flow_tasks, t.nseg, t.nnz_total, t.flow_far);
   } else if (t.seg) {
     snprintf(buf, sizeof(buf), "  %s: segmented, %d segments, %d CTAs, %d lanes per row, %d dependency levels\n", what,
              t.nseg, t.nblocks, t.S, t.nlevels);
@@ -1007,47 +857,31 @@ struct Engine : EngineBase {
 
   // dynamic shared memory of the per-subdomain solve for R right-hand sides
   template <int R>
-  static int set_pipe_smem() {
-    const int bytes = (int)PipeCfg<P, R>::bytes;
-#define PGX_PIPEATTR(SS)                                                                                     \
-  PGX_CUDA(cudaFuncSetAttribute(trsv_pipe_kernel<P, SS, false, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                bytes));                                                                     \
-  PGX_CUDA(cudaFuncSetAttribute(trsv_pipe_kernel<P, SS, true, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
-    PGX_PIPEATTR(2);
-    PGX_PIPEATTR(4);
-    PGX_PIPEATTR(8);
-    PGX_PIPEATTR(16);
-#undef PGX_PIPEATTR
+  static int set_flow_smem() {
+    using C = FlowCfg<P, R>;
+    const auto most = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    PGX_CUDA(cudaFuncSetAttribute(trsv_flow_kernel<P, false, R>, most, (int)C::bytes));
+    PGX_CUDA(cudaFuncSetAttribute(trsv_flow_kernel<P, true, R>, most, (int)C::bytes));
+    if constexpr (C::has_long) {
+      using L = FlowCfg<P, R, true>;
+      PGX_CUDA(cudaFuncSetAttribute(trsv_flow_kernel<P, false, R, L>, most, (int)L::bytes));
+      PGX_CUDA(cudaFuncSetAttribute(trsv_flow_kernel<P, true, R, L>, most, (int)L::bytes));
+    }
     return PGX_SUCCESS;
   }
 
   // the per-subdomain solve of factor T for R right-hand sides
-  template <int R>
-  static void launch_pipe(const DTri<P>& T, bool upper, const PtrR<P, R>& yslot, const PtrR<P, R>& rhs,
-                          const PtrR<P, R>& y, const PtrR<P, R>& x, int* err, const SkipR<R>& sk, cudaStream_t st) {
-    const size_t bytes = PipeCfg<P, R>::bytes;
-    CompArrays ca;
-    ca.meta = (const int4*)T.cmeta;
-    ca.ord = T.ord;
-    ca.rp = T.rp;
-    ca.cj = T.cj;
-    ca.lvb = T.lvb;
-    ca.uslot = T.uslot;
-    ca.far_col = T.far_col;
-#define PGX_PIPE(SS)                                                                                             \
-  if (upper)                                                                                                     \
-    trsv_pipe_kernel<P, SS, true, R><<<T.ncomp, kPipeThreads, bytes, st>>>(                                       \
-        T.n, T.nslots_up, T.comp_ch0, ca, T.va, T.dslot, yslot, rhs, y, x, err, sk);                               \
-  else                                                                                                           \
-    trsv_pipe_kernel<P, SS, false, R><<<T.ncomp, kPipeThreads, bytes, st>>>(                                      \
-        T.n, T.nslots_up, T.comp_ch0, ca, T.va, T.dslot, yslot, rhs, y, x, err, sk)
-    switch (T.S) {
-      case 2: PGX_PIPE(2); break;
-      case 4: PGX_PIPE(4); break;
-      case 8: PGX_PIPE(8); break;
-      default: PGX_PIPE(16); break;
+  template <int R, bool LONG = false>
+  static void launch_flow(const DTri<P>& T, bool upper, const PtrR<P, R>& yslot, const PtrR<P, R>& rhs,
+                          const PtrR<P, R>& x, int* err, const SkipR<R>& sk, cudaStream_t st) {
+    using C = FlowCfg<P, R, LONG>;
+    if constexpr (!LONG && C::has_long) {
+      if (T.flow_long) return launch_flow<R, true>(T, upper, yslot, rhs, x, err, sk, st);
     }
-#undef PGX_PIPE
+    if (upper)
+      trsv_flow_kernel<P, true, R, C><<<T.ncomp, C::threads, C::bytes, st>>>(T.flow, yslot, rhs, x, err, sk);
+    else
+      trsv_flow_kernel<P, false, R, C><<<T.ncomp, C::threads, C::bytes, st>>>(T.flow, yslot, rhs, x, err, sk);
   }
 
   int set_seg_smem() {
@@ -1061,7 +895,7 @@ struct Engine : EngineBase {
     PGX_SEGATTR(16);
     PGX_SEGATTR(32);
 #undef PGX_SEGATTR
-    PGX_TRY(set_pipe_smem<1>());
+    PGX_TRY(set_flow_smem<1>());
     return PGX_SUCCESS;
   }
 
@@ -1114,10 +948,11 @@ struct Engine : EngineBase {
       int rcL = PGX_ERROR_INVALID_PARAM, rcU = PGX_ERROR_INVALID_PARAM;
       if (h.L.rows > 0) {
         std::vector<int> uslot_of_row;
-        rcU = upload_tri_comp(ar, h.U, true, h.dom_ptr, d.U, stream, &h.dinv, &uslot_of_row, nullptr);
+        rcU = upload_tri_flow<P, 1>(ar, h.U, true, h.dom_ptr, d.U, stream, &h.dinv, &uslot_of_row, nullptr);
         if (rcU == PGX_SUCCESS)
-          rcL = upload_tri_comp(ar, h.L, false, h.dom_ptr, d.L, stream, nullptr, nullptr, &uslot_of_row);
-        d.L.nslots_up = d.U.nslots_up = d.U.nslots;
+          rcL = upload_tri_flow<P, 1>(ar, h.L, false, h.dom_ptr, d.L, stream, nullptr, nullptr, &uslot_of_row);
+        for (int rc : {rcU, rcL})
+          if (rc != PGX_SUCCESS && rc != PGX_ERROR_INVALID_PARAM) return rc;
       }
       if (rcL == PGX_SUCCESS && rcU == PGX_SUCCESS) {
         // one CTA per subdomain; y travels from the lower to the upper pass in slot order
@@ -1165,7 +1000,7 @@ struct Engine : EngineBase {
   int alloc_work() {
     for (int l = 0; l < nlev; l++) {
       DLevel<P>& d = lv[l];
-      if (d.L.comp) PGX_TRY(wk.zeros(&d.yslot, (size_t)d.U.nslots, stream));
+      if (d.L.comp) PGX_TRY(wk.zeros(&d.yslot, (size_t)d.nl, stream));
       if (!owner) {
         // the level-set and segmented kernels count their CTAs per slot
         if (d.L.ticket) PGX_TRY(wk.zeros(&d.L.ticket, 2, stream));
@@ -1512,14 +1347,13 @@ struct Engine : EngineBase {
             Skip sk, P* yslot = nullptr) {
     if (T.n == 0) return;
     if (T.comp) {
-      PtrR<P, 1> pys, prhs, py, px;
+      PtrR<P, 1> pys, prhs, px;
       pys.p[0] = yslot;
       prhs.p[0] = const_cast<P*>(rhs);
-      py.p[0] = y;
       px.p[0] = x;
       SkipR<1> sr;
       sr.s[0] = sk;
-      launch_pipe<1>(T, upper, pys, prhs, py, px, err, sr, stream);
+      launch_flow<1>(T, upper, pys, prhs, px, err, sr, stream);
       return;
     }
     if (T.seg) {
@@ -2320,7 +2154,7 @@ struct Engine : EngineBase {
 };
 
 // Per-level layout of the triangular factors for R right-hand sides at once
-// (the PipeCfg<P, R> chunking), built once per handle and read by every R-lane
+// (the FlowCfg<P, R> layout), built once per handle and read by every R-lane
 // slot.  Levels whose factors do not fit that layout keep each lane's own
 // single-right-hand-side kernels.
 template <typename P, int R>
@@ -2332,7 +2166,7 @@ struct BatchLayout {
 // A solve slot that advances R right-hand sides in lockstep: R lanes, each
 // with its own FGMRES state and work vectors (clones of the owner), share one
 // stream and one captured restart cycle.  The triangular passes of the
-// preconditioner are merged over the lanes (trsv_pipe_kernel with R lanes: each
+// preconditioner are merged over the lanes (trsv_flow_kernel with R lanes: each
 // factor entry is read once for R vectors); every other kernel runs once per
 // lane exactly as in Engine, so each lane's arithmetic is that of a single
 // solve and its result matches it bit for bit.
@@ -2383,7 +2217,7 @@ struct BatchEngine : EngineBase {
   }
 
   int setup(Engine<P>& own, Import& im, std::shared_ptr<BatchLayout<P, G>> shared) {
-    PGX_TRY(Engine<P>::template set_pipe_smem<G>());
+    PGX_TRY(Engine<P>::template set_flow_smem<G>());
     owner = &own;
     n = own.n;
     nlev = own.nlev;
@@ -2407,20 +2241,15 @@ struct BatchEngine : EngineBase {
         HostLevel& h = im.levels[l];
         if (h.L.rows == 0 || !own.lv[l].L.comp) continue;
         std::vector<int> uslot_of_row;
-        using CC = PipeCfg<P, G>;
-        int rc = upload_tri_sub<P, CC>(lay->ar, h.U, true, h.dom_ptr, lay->U[l], stream, &h.dinv, &uslot_of_row,
+        int rc = upload_tri_flow<P, G>(lay->ar, h.U, true, h.dom_ptr, lay->U[l], stream, &h.dinv, &uslot_of_row,
                                        nullptr);
         if (rc == PGX_SUCCESS)
-          rc = upload_tri_sub<P, CC>(lay->ar, h.L, false, h.dom_ptr, lay->L[l], stream, nullptr, nullptr,
+          rc = upload_tri_flow<P, G>(lay->ar, h.L, false, h.dom_ptr, lay->L[l], stream, nullptr, nullptr,
                                      &uslot_of_row);
-        lay->L[l].nslots_up = lay->U[l].nslots_up = lay->U[l].nslots;
+        if (rc != PGX_SUCCESS && rc != PGX_ERROR_INVALID_PARAM) return rc;
         if (rc != PGX_SUCCESS) {
           lay->L[l] = DTri<P>();
           lay->U[l] = DTri<P>();
-        } else {
-          // rows are summed as the handle's own slot sums them
-          lay->L[l].S = own.lv[l].L.S;
-          lay->U[l].S = own.lv[l].U.S;
         }
       }
     }
@@ -2428,7 +2257,7 @@ struct BatchEngine : EngineBase {
     for (int l = 0; l < nlev; l++)
       for (int r = 0; r < R; r++) {
         yslot[l][r] = nullptr;
-        if (lay->U[l].comp) PGX_TRY(wk.zeros(&yslot[l][r], (size_t)lay->U[l].nslots, stream));
+        if (lay->U[l].comp) PGX_TRY(wk.zeros(&yslot[l][r], (size_t)lay->U[l].n, stream));
       }
     for (int k = 0; k < NSIDE; k++) {
       PGX_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
@@ -2523,16 +2352,15 @@ struct BatchEngine : EngineBase {
       const int k = g0 / G - 1;  // side stream of this group (-1: the slot's own)
       cudaStream_t sg_stream = k < 0 ? stream : side[k];
       if (k >= 0) cudaStreamWaitEvent(sg_stream, ev_fork, 0);
-      PtrR<P, G> prhs, py, px, pys;
+      PtrR<P, G> prhs, px, pys;
       SkipR<G> sg;
       for (int r = 0; r < G; r++) {
         prhs.p[r] = const_cast<P*>(rhs[g0 + r]);
-        py.p[r] = y[g0 + r];
         px.p[r] = x[g0 + r];
         pys.p[r] = yslot[l][g0 + r];
         sg.s[r] = sk[g0 + r];
       }
-      Engine<P>::template launch_pipe<G>(T, upper, pys, prhs, py, px, lane[0]->err, sg, sg_stream);
+      Engine<P>::template launch_flow<G>(T, upper, pys, prhs, px, lane[0]->err, sg, sg_stream);
       if (k >= 0) cudaEventRecord(ev_join[k], sg_stream);
     }
     for (int k = 0; k < NSIDE; k++) cudaStreamWaitEvent(stream, ev_join[k], 0);

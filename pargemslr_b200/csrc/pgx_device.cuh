@@ -716,19 +716,8 @@ __global__ void __launch_bounds__(kSegThreads) trsv_seg_kernel(
   }
 }
 
-// ----------------------------- one-CTA-per-subdomain triangular solve
-// Same arithmetic as trsv_kernel.  In level-set order the dependencies of an
-// ILU factor are short-range: for the RCM-ordered subdomains of a 3D problem
-// the median distance between a row and the rows it needs is ~10^3
-// positions and almost all are within 10^4.  So one CTA walks a whole
-// subdomain (trsv_pipe_kernel below), for R right-hand sides at once.
-#ifndef PGX_PIPE_THREADS
-#define PGX_PIPE_THREADS 512
-#endif
-// one CTA per subdomain; the SM's other thread slots stay free for other kernels
-constexpr int kPipeThreads = PGX_PIPE_THREADS;
-constexpr int kPipeStages = 4;     // chunks in flight: the one being solved and three being staged
-constexpr int kUnroll = 4;         // operands per lane loaded before any is used
+// ------------------------------------------------ building blocks of the
+// one-CTA-per-subdomain triangular solve (pgx_flow.cuh)
 constexpr long long kMbarWaitCycles = 1ll << 31;  // bound of a wait on a staging barrier: about 1 s
 
 template <typename T, int R>
@@ -739,78 +728,6 @@ template <typename T, int R>
 struct PtrR {
   T* p[R];
 };
-
-// Shared-memory plan of the pipelined solve for value type T and R
-// right-hand sides: a ring of the last `ring` results (R values per schedule
-// position) followed by three far-operand buffers of `far` entries, then
-// kPipeStages staging buffers of one chunk each (at most `nnz` nonzeros and
-// `rows` rows, padding included).  Operand indices into the ring are checked
-// once on the host when the layout is built; the kernel clamps them into the
-// shared array, so a damaged layout can give wrong values but never an
-// access outside shared memory.
-template <typename T, int R>
-struct PipeCfg {
-  // sizes by value width: 4 bytes (FP32), 8 (FP64, complex64), 16 (complex128)
-  static constexpr bool d = sizeof(T) == 8;
-  static constexpr bool z = sizeof(T) == 16;
-  static constexpr int ring = z ? (R == 1 ? 4096 : R == 2 ? 2048 : 1024)
-                                : d ? (R == 1 ? 8192 : R == 2 ? 4096 : 2048) : (R == 4 ? 4096 : 8192);
-  static constexpr int far = z ? 256 : d ? (R == 1 ? 512 : 256) : 512;
-  static constexpr int nnz = z ? (R == 4 ? 768 : 1024)
-                               : d ? (R == 4 ? 1536 : 2048) : (R == 1 ? 4096 : R == 2 ? 3072 : 2560);
-  static constexpr int rows = z ? (R == 4 ? 128 : 192) : d ? 256 : (R == 1 ? 512 : R == 2 ? 384 : 320);
-  // per stage: va[nnz] T | sb[R][rows] T | sd[rows] T | cj[nnz] | ord[rows] | rp[rows+4] | lvb[rows+4] | fc[far]
-  static constexpr size_t buf_bytes =
-      sizeof(T) * (size_t)(nnz + (R + 1) * rows) + sizeof(int) * (size_t)(nnz + rows + 2 * (rows + 4) + far);
-  static constexpr size_t ring_bytes = sizeof(T) * R * (size_t)(ring + 3 * far);
-  static constexpr size_t bytes = ring_bytes + kPipeStages * buf_bytes;
-  static_assert(bytes <= 227 * 1024, "pipelined per-subdomain solve exceeds the shared memory of a CTA");
-  static_assert(far <= kPipeThreads && rows <= kPipeThreads, "one gather per thread");
-  static_assert((ring & (ring - 1)) == 0, "ring size must be a power of two");
-  static_assert(nnz % 4 == 0 && rows % 4 == 0 && far % 4 == 0 && buf_bytes % 16 == 0 && ring_bytes % 16 == 0,
-                "every staged array starts on a 16-byte boundary");
-};
-
-// Per-chunk metadata, two int4 per chunk: {row0, rp0, nnz0, lv0} and
-// {pos0, far0, 0, 0}: first slot of the chunk in the row list, the row
-// pointers, the nonzeros and the level boundaries; its first schedule
-// position; its first far operand.  One record past the last chunk closes the
-// ranges.  Every range starts on a 16-byte boundary and spans a multiple of
-// 16 bytes (padded on the host), so each is one bulk copy.
-struct ChunkMeta {
-  int row0, rp0, nnz0, lv0, pos0, far0;
-};
-__device__ __forceinline__ ChunkMeta load_meta(const int4* __restrict__ meta, int ch) {
-  const int4 a = __ldg(&meta[2 * ch]), b = __ldg(&meta[2 * ch + 1]);
-  ChunkMeta m;
-  m.row0 = a.x;
-  m.rp0 = a.y;
-  m.nnz0 = a.z;
-  m.lv0 = a.w;
-  m.pos0 = b.x;
-  m.far0 = b.y;
-  return m;
-}
-
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gmem_src) : "memory");
-}
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* dst, const T* src) {
-  if (sizeof(T) == 16) {
-    unsigned sd = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(sd), "l"(src) : "memory");
-  } else if (sizeof(T) == 8) {
-    cp_async8(dst, src);
-  } else {
-    cp_async4(dst, src);
-  }
-}
 
 // mbarrier and bulk-copy (TMA, non-tensor) helpers.  The copies read this
 // GPU's own global memory only.
@@ -849,302 +766,6 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
-}
-
-template <typename T, int R>
-struct PipeBuf {
-  T *va, *sb, *sd;  // sb: R arrays of `rows`; sd: inverse diagonal (upper) or upper-pass slots (lower, as int)
-  int *cj, *ord, *rp, *lvb, *fc;
-};
-template <typename T, int R, typename C = PipeCfg<T, R>>
-__device__ __forceinline__ PipeBuf<T, R> pipe_buf(unsigned char* base, int stage) {
-  unsigned char* b = base + C::ring_bytes + (size_t)stage * C::buf_bytes;
-  PipeBuf<T, R> o;
-  o.va = (T*)b;
-  o.sb = o.va + C::nnz;
-  o.sd = o.sb + R * C::rows;
-  o.cj = (int*)(o.sd + C::rows);
-  o.ord = o.cj + C::nnz;
-  o.rp = o.ord + C::rows;
-  o.lvb = o.rp + C::rows + 4;
-  o.fc = o.lvb + C::rows + 4;
-  return o;
-}
-
-struct CompArrays {
-  const int4* meta;
-  const int *ord, *rp, *cj, *lvb, *uslot, *far_col;
-};
-
-// one thread: stage chunk [m, me) into buffer b with bulk copies completing on
-// bar (the byte count is announced first)
-template <typename T, int R, bool UPPER>
-__device__ __forceinline__ void pipe_issue(const PipeBuf<T, R>& b, const ChunkMeta& m, const ChunkMeta& me,
-                                           const CompArrays& g, const T* __restrict__ va, const T* __restrict__ dslot,
-                                           const PtrR<T, R>& yslot, unsigned long long* bar) {
-  const unsigned nz = (unsigned)(me.nnz0 - m.nnz0), nr = (unsigned)(me.row0 - m.row0);
-  const unsigned np = (unsigned)(me.rp0 - m.rp0), nv = (unsigned)(me.lv0 - m.lv0), nf = (unsigned)(me.far0 - m.far0);
-  unsigned total = nz * (sizeof(T) + 4) + nr * 4 + np * 4 + nv * 4 + nf * 4 + nr * (UPPER ? sizeof(T) : 4);
-  if (UPPER) total += R * nr * (unsigned)sizeof(T);
-  mbar_arrive_expect_tx(bar, total);
-  if (nz) {
-    bulk_g2s(b.va, va + m.nnz0, nz * (unsigned)sizeof(T), bar);
-    bulk_g2s(b.cj, g.cj + m.nnz0, nz * 4, bar);
-  }
-  bulk_g2s(b.ord, g.ord + m.row0, nr * 4, bar);
-  bulk_g2s(b.rp, g.rp + m.rp0, np * 4, bar);
-  bulk_g2s(b.lvb, g.lvb + m.lv0, nv * 4, bar);
-  if (nf) bulk_g2s(b.fc, g.far_col + m.far0, nf * 4, bar);
-  if (UPPER) {
-    bulk_g2s(b.sd, dslot + m.row0, nr * (unsigned)sizeof(T), bar);
-#pragma unroll
-    for (int r = 0; r < R; r++) bulk_g2s(b.sb + r * PipeCfg<T, R>::rows, yslot.p[r] + m.row0, nr * (unsigned)sizeof(T), bar);
-  } else {
-    bulk_g2s(b.sd, g.uslot + m.row0, nr * 4, bar);
-  }
-}
-
-// One CTA per subdomain solves its rows level by level (the schedule of
-// IluClass::BuildLevels, ilu.cpp:832-1062, restricted to the subdomain),
-// for R right-hand sides at once: a lower pass y = L^-1 rhs or an upper pass
-// x = D U^-1 y.  Each staged factor entry is read once and applied to all R
-// vectors.  Results live in a shared-memory ring indexed by schedule
-// position, so a dependency on the last `ring` positions is a shared-memory
-// read (one vector load for the R values).  An older ("far") operand lies,
-// by construction on the host, before the start of the previous chunk: it
-// was published to global memory before that chunk began, so it is gathered
-// into the far buffer while the previous chunk is being solved.  Column
-// indices are encoded as -(index + 1) into the ring-plus-far array.
-//
-// The subdomain's schedule is cut into chunks.  One thread stages chunk
-// c + kPipeStages - 1 with bulk copies (completing on that stage's mbarrier)
-// as soon as chunk c - 1 is done, so the factor streams in well ahead of the
-// solve; at the start of chunk c the CTA gathers what needs an index (the
-// lower pass's right-hand side through the row list, the far operands) for
-// chunk c + 1.  A chunk's end coincides with the barrier of its last level:
-// a chunk boundary costs no barrier of its own.  Each row's writing lanes
-// publish its result to global memory at once (natural order, and the upper
-// pass's slot order in the lower pass).  No CTA waits on another.
-template <typename T, int S, bool UPPER, int R, typename C = PipeCfg<T, R>>
-__global__ void __launch_bounds__(kPipeThreads, 1) trsv_pipe_kernel(
-    int n, int nslots, const int* __restrict__ comp_ch0, CompArrays g, const T* __restrict__ va,
-    const T* __restrict__ dslot, PtrR<T, R> yslot, PtrR<T, R> rhs, PtrR<T, R> y, PtrR<T, R> x, int* err,
-    SkipR<R> skip) {
-  // a wait of an earlier pass of this solve gave up: the solve reports the
-  // timeout, and the passes after it do no work
-  if (skip.on() || (*(volatile int*)err & (kErrTimeout | kErrStage))) return;
-  using V = VecR<T, R>;
-  constexpr int RF = C::ring + 3 * C::far;
-  constexpr int D = kPipeStages;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long s_full[D];
-  __shared__ ChunkMeta s_meta[D][2];  // {chunk, next chunk} of the chunk in each stage
-  __shared__ int s_abort;
-  V* ring = (V*)smem_raw;  // ring, then far buffers 0, 1, 2
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int c0 = comp_ch0[blockIdx.x], c1 = comp_ch0[blockIdx.x + 1];
-  const PtrR<T, R> out = UPPER ? x : y;
-  if (c0 >= c1) return;
-  // tid 0 keeps the metadata of the next chunk to stage and of the one after
-  ChunkMeta ma{}, mb{};
-  unsigned long long issued = 0, waited = 0;  // per-stage use counts, 16 bits each (tid 0), for the exit path
-  if (tid == 0) {
-    s_abort = 0;
-    for (int s = 0; s < D; s++) mbar_init(&s_full[s], 1);
-    mbar_fence_init();
-    ma = load_meta(g.meta, c0);
-    for (int k = 0; k < D && c0 + k < c1; k++) {
-      mb = load_meta(g.meta, c0 + k + 1);
-      s_meta[k][0] = ma;
-      s_meta[k][1] = mb;
-      pipe_issue<T, R, UPPER>(pipe_buf<T, R>(smem_raw, k), ma, mb, g, va, dslot, yslot, &s_full[k]);
-      issued += 1ull << (16 * k);
-      ma = mb;
-    }
-    mb = c0 + D + 1 <= c1 ? load_meta(g.meta, c0 + D + 1) : ma;
-  }
-  __syncthreads();
-  const int sl = tid & (S - 1), group = tid / S;
-  constexpr int NG = kPipeThreads / S;
-  // What needs an index is gathered two chunks ahead, into chunk j's stage
-  // (the lower pass's right-hand side through the row list) and into far
-  // buffer j % 3 (the far operands, which the host placed before the start
-  // of chunk j - 2, so they are published by then); each chunk's gathers are
-  // one cp.async group.
-  auto gather = [&](int j) {  // j: chunk index within the subdomain
-    const int sj = j % D;
-    if (!mbar_wait(&s_full[sj], (unsigned)((j / D) & 1), err)) {
-      s_abort = 1;  // the staged indices are not there: gather nothing
-      return;
-    }
-    if (tid == 0) waited += 1ull << (16 * sj);
-    const PipeBuf<T, R> nb = pipe_buf<T, R>(smem_raw, sj);
-    const ChunkMeta n0 = s_meta[sj][0], n1 = s_meta[sj][1];
-    if (!UPPER && tid < n1.row0 - n0.row0) {
-      const int rr = nb.ord[tid];
-      if ((unsigned)rr < (unsigned)n) {
-#pragma unroll
-        for (int r = 0; r < R; r++) cp_async_elem(&nb.sb[r * C::rows + tid], &rhs.p[r][rr]);
-      } else if (rr >= 0) {
-        atomicOr(err, kErrIndex);
-      }
-    }
-    if (tid < n1.far0 - n0.far0) {
-      const int fcol = nb.fc[tid];
-      if ((unsigned)fcol < (unsigned)n) {
-        V* fv = &ring[C::ring + (j % 3) * C::far + tid];
-#pragma unroll
-        for (int r = 0; r < R; r++) cp_async_elem(&fv->v[r], &out.p[r][fcol]);
-      } else if (fcol >= 0) {
-        atomicOr(err, kErrIndex);
-      }
-    }
-  };
-  gather(0);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  if (c0 + 1 < c1) gather(1);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("cp.async.wait_group 1;" ::: "memory");
-  __syncthreads();
-  for (int ch = c0; ch < c1; ch++) {
-    if (s_abort) break;
-    const int k = ch - c0;
-    const int st = k % D;
-    const PipeBuf<T, R> b = pipe_buf<T, R>(smem_raw, st);
-    const ChunkMeta m0 = s_meta[st][0], m1 = s_meta[st][1];
-    if (ch + 2 < c1) gather(k + 2);
-    asm volatile("cp.async.commit_group;" ::: "memory");  // (empty near the end: keeps one group per chunk)
-    const int pos0 = m0.pos0;
-    const int nl = m1.lv0 - m0.lv0;
-    // Every read of this chunk's stage happens before the barrier of its
-    // last level: right after that barrier thread 0 reuses the stage for
-    // the chunk kPipeStages ahead, so the boundary of the next level is read
-    // before each barrier, and the last level ends the loop.
-    int a = b.lvb[0];
-    int e = nl > 1 ? b.lvb[1] : a;
-    if (a >= e) {  // no level (the host never builds such a chunk): still land the gathers
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      __syncthreads();
-    }
-    for (int lv = 0; a < e; lv++) {
-      for (int i = a + group; i < e; i += NG) {
-        // row pointers stay inside the staged nonzeros
-        const int k1 = max(b.rp[i], 0), k2 = min(b.rp[i + 1], C::nnz);
-        T acc[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) acc[r] = 0;
-        int q[kUnroll];
-        T v[kUnroll];
-#pragma unroll
-        for (int u = 0; u < kUnroll; u++) {
-          const int kk = k1 + sl + u * S;
-          q[u] = kk < k2 ? -b.cj[kk] - 1 : 0;
-          v[u] = kk < k2 ? b.va[kk] : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; u++) {
-          if (k1 + sl + u * S < k2) {  // never read an unwritten ring slot
-            const V w = ring[min((unsigned)q[u], (unsigned)(RF - 1))];
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r] += v[u] * w.v[r];
-          }
-        }
-        for (int kk = k1 + sl + kUnroll * S; kk < k2; kk += S) {
-          const int qq = -b.cj[kk] - 1;
-          const V w = ring[min((unsigned)qq, (unsigned)(RF - 1))];
-          const T vv = b.va[kk];
-#pragma unroll
-          for (int r = 0; r < R; r++) acc[r] += vv * w.v[r];
-        }
-        // sum over the group's lanes for every right-hand side: for R > 1 a
-        // reduce-scatter first (each step halves the values a lane carries),
-        // then a butterfly on one value.  Every partial sum adds the same two
-        // operands as group_reduce does, so the results are identical to the
-        // one-right-hand-side solve's.  Each result is written by one lane:
-        // into the ring and, at once, to global memory.
-        const unsigned gmask = S == 32 ? 0xffffffffu : (((1u << S) - 1u) << (lane & ~(S - 1)));
-        auto put = [&](int r, T o) {
-          const T bb = b.sb[r * C::rows + i];
-          const T res = UPPER ? (bb - o) * b.sd[i] : bb - o;
-          ring[(pos0 + i) & (C::ring - 1)].v[r] = res;
-          // pick the lane's pointers by comparison: no dynamic index into a
-          // parameter array (that would go through local memory)
-          T* op = out.p[0];
-          T* ys = yslot.p[0];
-#pragma unroll
-          for (int rr = 1; rr < R; rr++)
-            if (rr == r) {
-              op = out.p[rr];
-              ys = yslot.p[rr];
-            }
-          const int orow = b.ord[i];
-          if ((unsigned)orow < (unsigned)n)
-            op[orow] = res;
-          else
-            atomicOr(err, kErrIndex);
-          if (!UPPER) {
-            const int us = ((const int*)b.sd)[i];
-            if ((unsigned)us < (unsigned)nslots)
-              ys[us] = res;
-            else
-              atomicOr(err, kErrIndex);
-          }
-        };
-        if constexpr (R == 4 && S >= 4) {
-          const bool hb = (sl & (S >> 1)) != 0, qb = (sl & (S >> 2)) != 0;
-          T k0 = hb ? acc[2] : acc[0], kx = hb ? acc[3] : acc[1];
-          const T s0 = hb ? acc[0] : acc[2], s1 = hb ? acc[1] : acc[3];
-          k0 += __shfl_xor_sync(gmask, s0, S >> 1);
-          kx += __shfl_xor_sync(gmask, s1, S >> 1);
-          T kk = qb ? kx : k0;
-          kk += __shfl_xor_sync(gmask, qb ? k0 : kx, S >> 2);
-#pragma unroll
-          for (int off = S >> 3; off > 0; off >>= 1) kk += __shfl_xor_sync(gmask, kk, off);
-          if ((sl & ((S >> 2) - 1)) == 0) put((hb ? 2 : 0) + (qb ? 1 : 0), kk);
-        } else if constexpr (R == 2 && S >= 2) {
-          const bool hb = (sl & (S >> 1)) != 0;
-          T kk = hb ? acc[1] : acc[0];
-          kk += __shfl_xor_sync(gmask, hb ? acc[0] : acc[1], S >> 1);
-#pragma unroll
-          for (int off = S >> 2; off > 0; off >>= 1) kk += __shfl_xor_sync(gmask, kk, off);
-          if ((sl & ((S >> 1) - 1)) == 0) put(hb ? 1 : 0, kk);
-        } else {
-#pragma unroll
-          for (int r = 0; r < R; r++) acc[r] = group_reduce(acc[r], S, lane);
-          if (sl == 0) {
-#pragma unroll
-            for (int r = 0; r < R; r++) put(r, acc[r]);
-          }
-        }
-      }
-      // the next boundary (the padding after the last one repeats it)
-      const int e2 = lv + 2 < nl ? b.lvb[lv + 2] : e;
-      // the last level of the chunk: the next chunk's gathers (all groups but
-      // the newest) have landed before the barrier
-      if (e2 <= e) asm volatile("cp.async.wait_group 1;" ::: "memory");
-      __syncthreads();
-      a = e;
-      e = e2;
-    }
-    // chunk done: its stage is free for the chunk kPipeStages ahead
-    if (tid == 0 && ch + D < c1) {
-      s_meta[st][0] = ma;
-      s_meta[st][1] = mb;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      pipe_issue<T, R, UPPER>(b, ma, mb, g, va, dslot, yslot, &s_full[st]);
-      issued += 1ull << (16 * st);
-      ma = mb;
-      if (ch + D + 2 <= c1) mb = load_meta(g.meta, ch + D + 2);
-    }
-  }
-  if (s_abort && tid == 0) {
-    // a staging wait gave up: let the copies still in flight land (bounded)
-    // before the CTA's shared memory is released
-    for (int s = 0; s < D; s++) {
-      const unsigned is = (unsigned)(issued >> (16 * s)) & 0xffffu, ws = (unsigned)(waited >> (16 * s)) & 0xffffu;
-      for (unsigned u = ws; u < is; u++) mbar_wait(&s_full[s], u & 1u, err);
-    }
-  }
 }
 
 // ------------------------------------------------- tall-skinny kernels

@@ -1,0 +1,79 @@
+"""The per-subdomain triangular solve at the edges of its tasks, groups and ring, against plain substitution."""
+import numpy as np
+import pytest
+
+from pargemslr_b200.structures import GemslrStructures, LevelStructures, empty_csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _factors(dom, deg, back, seed, cplx, longrow=0):
+    """A random factor pair, block diagonal over `dom`: up to `deg` entries a row, at most `back` rows away."""
+    rng = np.random.default_rng(seed)
+    n = dom[-1]
+    out = []
+    for up in (False, True):
+        rp, cj = [0], []
+        for a, e in zip(dom[:-1], dom[1:]):
+            for i in range(a, e):
+                room = e - 1 - i if up else i - a
+                want = min(room, longrow if longrow and i % 97 == 96 else int(rng.integers(0, deg + 1)))
+                d = np.unique(1 + rng.integers(0, min(room, max(back, want)), want)) if want else np.zeros(0, np.int64)
+                cj.append(np.sort(i + d if up else i - d))
+                rp.append(rp[-1] + len(d))
+        cj = np.concatenate(cj).astype(np.int32)
+        rp = np.array(rp, np.int32)
+        va = rng.uniform(-1, 1, len(cj)) / (1.0 + np.repeat(np.diff(rp), np.diff(rp)))
+        if cplx:
+            va = va + 1j * rng.uniform(-1, 1, len(cj)) / 4
+        out.append((rp, cj, va, n, n))
+    return out[0], out[1], 1.0 + 0.2 * rng.uniform(-1, 1, n) + (0.1j if cplx else 0.0)
+
+
+def _substitute(L, U, dinv, b):
+    y = b.astype(np.result_type(b, dinv))
+    for M, up in ((L, False), (U, True)):
+        rp, cj, va = M[:3]
+        for i in (range(len(b) - 1, -1, -1) if up else range(len(b))):
+            y[i] -= va[rp[i]:rp[i + 1]] @ y[cj[rp[i]:rp[i + 1]]]
+            if up:
+                y[i] *= dinv[i]
+    return y
+
+
+CASES = {
+    "one row": ([0, 1], 0, 1, 0),
+    "a task and a row": ([0, 33], 3, 20, 0),
+    "diagonal": ([0, 1300], 0, 1, 0),
+    "chain": ([0, 400], 1, 1, 0),
+    "two narrow subdomains and an empty one": ([0, 517, 517, 900], 6, 40, 0),
+    "long rows": ([0, 2500], 6, 150, 90),
+    "ring wraps": ([0, 20000], 4, 30, 0),
+    "operands older than the ring": ([0, 24000], 4, 9000, 0),
+}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+@pytest.mark.parametrize("name", CASES)
+def test_pass_pair(name, cplx, precision):
+    from pargemslr_b200.handle import GemslrHandle
+    dom, deg, back, longrow = CASES[name]
+    L, U, dinv = _factors(dom, deg, back, len(name), cplx, longrow)
+    n = dom[-1]
+    eye = (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n, dinv.dtype), n, n)
+    lv = LevelStructures(ncomp=len(dom) - 1, dom_ptr=np.array(dom, np.int32), L=L, U=U, dinv=dinv, B=eye)
+    st = GemslrStructures(n=n, A=eye, pperm=np.arange(n, dtype=np.int32), qperm=None,
+                          lev_ptr=np.array([0, n], np.int32), levels=[lv], inner_enable=0)
+    rng = np.random.default_rng(1)
+    b = rng.standard_normal(n) + (1j * rng.standard_normal(n) if cplx else 0.0)
+    h = GemslrHandle(st, precision=precision)
+    try:
+        assert "dataflow" in h.describe()
+        z = h.apply(b)
+    finally:
+        h.close()
+    ref = _substitute(L, U, dinv, b)
+    # |x| stays of order |b| (row sums of the factors are below 1): rounding of 90 products a row at most
+    tol = 1e-13 if precision == "fp64" else 2e-5
+    assert np.linalg.norm(z - ref) <= tol * np.linalg.norm(ref)
