@@ -304,6 +304,48 @@ struct Arena {
   }
 };
 
+// Scratch of a call that runs on the legacy stream (calls without a handle),
+// from one memory pool per device.  The pool keeps at most kScratchKeep bytes
+// between calls, hands memory out in stream order, so several threads may
+// use it, and gives everything back in pgx_finalize.
+constexpr uint64_t kScratchKeep = 32ull << 20;
+static std::mutex g_scratch_mutex;
+static cudaMemPool_t g_scratch_pool[64] = {};
+static int scratch_pool(cudaMemPool_t* out) {
+  int dev = 0;
+  PGX_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return fail(PGX_ERROR_NO_DEVICE, "device %d", dev);
+  std::lock_guard<std::mutex> lock(g_scratch_mutex);
+  if (!g_scratch_pool[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    PGX_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = kScratchKeep;
+    PGX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    g_scratch_pool[dev] = pool;
+  }
+  *out = g_scratch_pool[dev];
+  return PGX_SUCCESS;
+}
+struct Scratch {
+  void* p = nullptr;
+  Scratch() {}
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  ~Scratch() {
+    if (p) cudaFreeAsync(p, 0);
+  }
+  int take(size_t bytes) {
+    cudaMemPool_t pool = nullptr;
+    PGX_TRY(scratch_pool(&pool));
+    PGX_CUDA(cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 16), pool, 0));
+    return PGX_SUCCESS;
+  }
+};
+
 template <typename T>
 struct DCsr {
   int rows = 0, cols = 0, S = 8;
@@ -3445,7 +3487,12 @@ int pgx_init(int device) {
   return PGX_SUCCESS;
 }
 
-int pgx_finalize(void) { return PGX_SUCCESS; }
+int pgx_finalize(void) {
+  std::lock_guard<std::mutex> lock(g_scratch_mutex);
+  for (cudaMemPool_t pool : g_scratch_pool)
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+  return PGX_SUCCESS;
+}
 
 const char* pgx_last_error(void) { return g_last_error.c_str(); }
 
@@ -4641,51 +4688,43 @@ int pgx_csr_spmv_device_variant(const pgx_csr* Ad, int32_t variant, double alpha
     if (Ad->rows == 0) return PGX_SUCCESS;
     if (Ad->nnz > INT32_MAX || (long long)Ad->rows + Ad->nnz > INT32_MAX)
       return fail(PGX_ERROR_INVALID_PARAM, "matrix too large for 32-bit indices");
-    // the plan needs the row pointer on the host
-    std::vector<int> rp(Ad->rows + 1);
-    PGX_CUDA(cudaMemcpy(rp.data(), Ad->rowptr, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost));
-    const SpmvPlan p = spmv_plan(Ad->rows, rp.data());
-    const bool merge = variant == 2 || (variant == 0 && p.merge);
-    Skip sk = mk_skip();
     const double* b = beta != 0.0 ? y : nullptr;
-    if (merge) {
+    auto merge_path = [&]() -> int {
       const int nt = merge_threads(Ad->rows, Ad->nnz);
-      Arena tmp;
-      int* crow = nullptr;
-      double* cval = nullptr;
-      PGX_TRY(tmp.alloc(&crow, (size_t)nt));
-      PGX_TRY(tmp.alloc(&cval, (size_t)nt));
+      Scratch carry;
+      PGX_TRY(carry.take((size_t)nt * (sizeof(double) + sizeof(int))));
+      double* cval = (double*)carry.p;
+      int* crow = (int*)(cval + nt);
       merge_spmv_kernel<double, double, double, double><<<(nt + 255) / 256, 256>>>(
-          Ad->rows, (int)Ad->nnz, Ad->rowptr, Ad->colidx, Ad->values, x, alpha, b, beta, y, crow, cval, sk);
-      merge_spmv_fixup_kernel<double, double><<<grid_for(nt, 256, num_sms() * 8), 256>>>(nt, crow, cval, alpha, y, sk);
+          Ad->rows, (int)Ad->nnz, Ad->rowptr, Ad->colidx, Ad->values, x, alpha, b, beta, y, crow, cval, mk_skip());
+      merge_spmv_fixup_kernel<double, double>
+          <<<grid_for(nt, 256, num_sms() * 8), 256>>>(nt, crow, cval, alpha, y, mk_skip());
       PGX_CUDA(cudaGetLastError());
       PGX_CUDA(cudaDeviceSynchronize());
       return PGX_SUCCESS;
-    }
-    const int S = p.S;
-    const int grid = grid_for(Ad->rows, 256 / S, num_sms() * 16);
+    };
+    if (variant == 2) return merge_path();
+    Scratch mem;
+    PGX_TRY(mem.take(sizeof(SpmvPlanDev)));
+    SpmvPlanDev* plan = (SpmvPlanDev*)mem.p;
+    PGX_CUDA(cudaMemsetAsync(plan, 0, sizeof(SpmvPlanDev), 0));
+    spmv_plan_kernel<<<grid_for(Ad->rows, 1024, num_sms() * 2), 512>>>(Ad->rows, Ad->nnz, Ad->rowptr, plan);
+    // the plan is not known here: blocks for eight lanes a row (fewer lanes leave some of them nothing to do)
+    const int grid = grid_for(Ad->rows, 32, num_sms() * 16);
     // caller-owned arrays: 128-bit loads only where both are 16-byte aligned
     // and the nonzeros fill whole 4-entry blocks
     const bool vec = ((uintptr_t)Ad->colidx % 16 == 0) && ((uintptr_t)Ad->values % 16 == 0) && Ad->nnz % 4 == 0;
-#define PGX_SPMV1(SS)                                                                                             \
-  if (vec)                                                                                                        \
-    spmv_kernel<double, double, double, double, SS, true><<<grid, 256>>>(                                         \
-        Ad->rows, Ad->rowptr, Ad->colidx, Ad->values, x, Ad->cols, alpha, nullptr, nullptr, nullptr, nullptr, 0, \
-        0.0, b, beta, y, nullptr, nullptr, sk);                                                                   \
-  else                                                                                                            \
-    spmv_kernel<double, double, double, double, SS, false><<<grid, 256>>>(                                        \
-        Ad->rows, Ad->rowptr, Ad->colidx, Ad->values, x, Ad->cols, alpha, nullptr, nullptr, nullptr, nullptr, 0, \
-        0.0, b, beta, y, nullptr, nullptr, sk)
-    switch (S) {
-      case 2: PGX_SPMV1(2); break;
-      case 4: PGX_SPMV1(4); break;
-      case 8: PGX_SPMV1(8); break;
-      case 16: PGX_SPMV1(16); break;
-      default: PGX_SPMV1(32); break;
-    }
-#undef PGX_SPMV1
+    if (vec)
+      spmv_planned_kernel<true><<<grid, 256>>>(plan, variant == 1, Ad->rows, Ad->rowptr, Ad->colidx, Ad->values, x,
+                                               Ad->cols, alpha, b, beta, y);
+    else
+      spmv_planned_kernel<false><<<grid, 256>>>(plan, variant == 1, Ad->rows, Ad->rowptr, Ad->colidx, Ad->values, x,
+                                                Ad->cols, alpha, b, beta, y);
     PGX_CUDA(cudaGetLastError());
+    int chosen[2] = {0, 0};  // S, merge
+    PGX_CUDA(cudaMemcpyAsync(chosen, &plan->S, sizeof(chosen), cudaMemcpyDeviceToHost, 0));
     PGX_CUDA(cudaDeviceSynchronize());
+    if (variant == 0 && chosen[1]) return merge_path();
     return PGX_SUCCESS;
   });
 }

@@ -243,12 +243,11 @@ __device__ __forceinline__ TC row_dot_vec(int k1, int k2, int lane, const int* _
 }
 
 template <typename TA, typename TX, typename TY, typename TC, int S, bool VEC>
-__global__ void __launch_bounds__(256) spmv_kernel(
+__device__ __forceinline__ void spmv_rows(
     int nrows, const int* __restrict__ rp1, const int* __restrict__ cj1, const TA* __restrict__ va1,
     const TX* __restrict__ x1, int xcols1, TC alpha, const int* __restrict__ rp2, const int* __restrict__ cj2,
     const TA* __restrict__ va2, const TX* __restrict__ x2, int xcols2, TC alpha2, const TY* b, TC beta, TY* y,
-    const double* __restrict__ xscale, int* err, Skip skip) {
-  if (skip.on()) return;
+    const double* __restrict__ xscale, int* err) {
   const int lane = threadIdx.x & (S - 1);
   const int wlane = threadIdx.x & 31;
   const int groups_per_block = blockDim.x / S;
@@ -275,6 +274,111 @@ __global__ void __launch_bounds__(256) spmv_kernel(
     }
   }
   if (bad && err) atomicOr(err, kErrIndex);
+}
+
+template <typename TA, typename TX, typename TY, typename TC, int S, bool VEC>
+__global__ void __launch_bounds__(256) spmv_kernel(
+    int nrows, const int* __restrict__ rp1, const int* __restrict__ cj1, const TA* __restrict__ va1,
+    const TX* __restrict__ x1, int xcols1, TC alpha, const int* __restrict__ rp2, const int* __restrict__ cj2,
+    const TA* __restrict__ va2, const TX* __restrict__ x2, int xcols2, TC alpha2, const TY* b, TC beta, TY* y,
+    const double* __restrict__ xscale, int* err, Skip skip) {
+  if (skip.on()) return;
+  spmv_rows<TA, TX, TY, TC, S, VEC>(nrows, rp1, cj1, va1, x1, xcols1, alpha, rp2, cj2, va2, x2, xcols2, alpha2, b, beta,
+                                    y, xscale, err);
+}
+
+// ------------------------------------------------- the variant of a matrix
+// whose arrays are on the device (pgx_csr_spmv_device).  spmv_plan_kernel
+// gathers what the rule of the host's spmv_plan asks of the row lengths, in
+// one pass over the row pointer: how many rows fit each batch size, the
+// longest row, and the nonzeros in rows longer than four batches; the last
+// block to finish applies the rule.  All sums are of integers, so the plan
+// is the host's.  spmv_planned_kernel then takes S from device memory, and
+// leaves a matrix planned for the merge path alone.
+// Bound by launches at small sizes and the row pointer's bytes at large ones.
+// On a B200, a whole pgx_csr_spmv_device call (plan, product, wait): 33 us at
+// 65,536 rows of a 5-point stencil and 83 us at 2,097,152 of a 7-point one;
+// with the row pointer copied to the host and planned there 196 us and 6.3 ms.
+constexpr int kPlanSizes = 5;  // S = 2, 4, 8, 16, 32
+struct SpmvPlanDev {
+  unsigned long long heavy[kPlanSizes];  // nonzeros of rows longer than 4 batches of S = 2 << k lanes
+  unsigned fits[kPlanSizes];             // rows of at most one batch
+  unsigned longest, blocks;              // the longest row; blocks that are done
+  int S, merge;
+};
+__global__ void __launch_bounds__(512) spmv_plan_kernel(int nrows, long long nnz, const int* __restrict__ rp,
+                                                        SpmvPlanDev* __restrict__ plan) {
+  __shared__ unsigned long long s_heavy[kPlanSizes];
+  __shared__ unsigned s_fits[kPlanSizes], s_longest;
+  if (threadIdx.x < kPlanSizes) {
+    s_heavy[threadIdx.x] = 0;
+    s_fits[threadIdx.x] = 0;
+  }
+  if (threadIdx.x == 0) s_longest = 0;
+  __syncthreads();
+  unsigned long long heavy[kPlanSizes] = {};
+  unsigned fits[kPlanSizes] = {}, longest = 0;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x) {
+    const int len = __ldg(&rp[r + 1]) - __ldg(&rp[r]);
+    longest = max(longest, (unsigned)max(len, 0));
+#pragma unroll
+    for (int k = 0; k < kPlanSizes; k++) {
+      const int batch = (2 << k) * kSpmvUnroll;
+      fits[k] += len <= batch;
+      if (len > 4 * batch) heavy[k] += (unsigned)len;
+    }
+  }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+#pragma unroll
+  for (int k = 0; k < kPlanSizes; k++) {
+    fits[k] = __reduce_add_sync(0xffffffffu, fits[k]);
+    heavy[k] = warp_reduce(heavy[k]);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_longest, longest);
+#pragma unroll
+    for (int k = 0; k < kPlanSizes; k++) {
+      atomicAdd(&s_fits[k], fits[k]);
+      if (heavy[k]) atomicAdd(&s_heavy[k], heavy[k]);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  atomicMax(&plan->longest, s_longest);
+  for (int k = 0; k < kPlanSizes; k++) {
+    atomicAdd(&plan->fits[k], s_fits[k]);
+    if (s_heavy[k]) atomicAdd(&plan->heavy[k], s_heavy[k]);
+  }
+  __threadfence();
+  if (atomicAdd(&plan->blocks, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  // the rows below and at the 90th percentile; k: the smallest size whose batch holds them
+  const unsigned want = (unsigned)min((long long)nrows, max(1ll, (long long)ceil(0.9 * nrows)));
+  int k = 0;
+  while (k < kPlanSizes - 1 && atomicAdd(&plan->fits[k], 0u) < want) k++;
+  const unsigned batch = (2u << k) * kSpmvUnroll;
+  plan->S = 2 << k;
+  plan->merge = atomicMax(&plan->longest, 0u) > 16 * batch && (long long)atomicAdd(&plan->heavy[k], 0ull) * 10 > nnz;
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(256) spmv_planned_kernel(const SpmvPlanDev* __restrict__ plan, int forced, int nrows,
+                                                           const int* __restrict__ rp, const int* __restrict__ cj,
+                                                           const double* __restrict__ va, const double* __restrict__ x,
+                                                           int xcols, double alpha, const double* b, double beta,
+                                                           double* y) {
+  if (plan->merge && !forced) return;
+#define PGX_ROWS(SS)                                                                                                   \
+  spmv_rows<double, double, double, double, SS, VEC>(nrows, rp, cj, va, x, xcols, alpha, nullptr, nullptr, nullptr,    \
+                                                     nullptr, 0, 0.0, b, beta, y, nullptr, nullptr)
+  switch (plan->S) {
+    case 2: PGX_ROWS(2); break;
+    case 4: PGX_ROWS(4); break;
+    case 8: PGX_ROWS(8); break;
+    case 16: PGX_ROWS(16); break;
+    default: PGX_ROWS(32); break;
+  }
+#undef PGX_ROWS
 }
 
 // ---------------------------------------------------- merge-path CSR SpMV
