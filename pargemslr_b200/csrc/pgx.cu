@@ -2966,6 +2966,9 @@ struct Systems : SystemsBase {
   int *d_ints = nullptr, *d_order = nullptr;
   P* d_p = nullptr;
   double* d_d = nullptr;
+  unsigned char* d_images = nullptr;
+  int* d_err = nullptr;
+  int* h_err = nullptr;  // pinned
   SysDesc<P>* d_desc = nullptr;
   double *d_bpack = nullptr, *d_xpack = nullptr;
   double *h_bpack = nullptr, *h_xpack = nullptr;  // pinned
@@ -2989,6 +2992,7 @@ struct Systems : SystemsBase {
     if (h_bpack) cudaFreeHost(h_bpack);
     if (h_xpack) cudaFreeHost(h_xpack);
     if (h_res) cudaFreeHost(h_res);
+    if (h_err) cudaFreeHost(h_err);
     if (h_bptr) cudaFreeHost(h_bptr);
     if (h_xptr) cudaFreeHost(h_xptr);
     if (ev0) cudaEventDestroy(ev0);
@@ -2998,12 +3002,14 @@ struct Systems : SystemsBase {
 
   struct Fix {
     void* field;
-    int kind;  // 0 ints, 1 P values, 2 doubles
+    int kind;  // 0 ints, 1 P values, 2 doubles, 3 task images
     size_t off;
   };
   std::vector<int> iv;
   std::vector<P> pv;
   std::vector<double> dv;
+  std::vector<unsigned char> images;
+  static constexpr int kSysFlowLevels = 8;
   std::vector<Fix> fix;
   static size_t padded(size_t n) { return (n + 63) / 64 * 64; }
   template <typename T, typename V>
@@ -3096,6 +3102,26 @@ struct Systems : SystemsBase {
     vals(&t.hva, hva.data(), hva.size());
     ints(&t.dst, dst.data(), dst.size());
     if (upper) vals(&t.dinv, di.data(), di.size());
+    // Task images for factors of at least kSysFlowLevels levels.  A flow pass
+    // takes about 4 us before its first row is out (barriers, ring, first
+    // chunk, first right-hand sides), a packed pass 0.7 us a level.  The
+    // separators of these systems have one to three levels, their subdomains
+    // hundreds.
+    t.nchunks = 0;
+    if (t.nlev >= kSysFlowLevels) {
+      FlowPack<P> pk;
+      auto val = [&](int k) { return (P)h.va[k]; };
+      auto diag = [&](int i) { return (P)(*dinv)[i]; };
+      if (flow_pack<P, SysFlowCfg<P>>(nl, h.rp.data(), h.cj.data(), val, upper, {0, nl}, &diag, dst_map, pk)) {
+        t.nchunks = (int)pk.chunk.size() / 4;
+        ints(&t.chunk, pk.chunk.data(), pk.chunk.size());
+        ints(&t.first, pk.first.data(), pk.first.size());
+        const size_t at = images.size();
+        images.insert(images.end(), pk.blob.begin(), pk.blob.end());
+        images.resize((images.size() + 255) / 256 * 256, 0);
+        fix.push_back({(void*)&t.blob, 3, at});
+      }
+    }
     if (pos_out) pos_out->swap(pos);
     return PGX_SUCCESS;
   }
@@ -3182,13 +3208,18 @@ struct Systems : SystemsBase {
     PGX_TRY(ar.upload(&d_ints, iv.data(), iv.size(), stream));
     PGX_TRY(ar.upload(&d_p, pv.data(), pv.size(), stream));
     PGX_TRY(ar.upload(&d_d, dv.data(), dv.size(), stream));
+    PGX_TRY(ar.upload(&d_images, images.data(), images.size(), stream));
     for (const Fix& f : fix) {
-      void* p = f.kind == 0 ? (void*)(d_ints + f.off) : f.kind == 1 ? (void*)(d_p + f.off) : (void*)(d_d + f.off);
+      void* p = f.kind == 0   ? (void*)(d_ints + f.off)
+                : f.kind == 1 ? (void*)(d_p + f.off)
+                : f.kind == 2 ? (void*)(d_d + f.off)
+                              : (void*)(d_images + f.off);
       *(void**)f.field = p;
     }
     iv.clear(), iv.shrink_to_fit();
     pv.clear(), pv.shrink_to_fit();
     dv.clear(), dv.shrink_to_fit();
+    images.clear(), images.shrink_to_fit();
     fix.clear();
     PGX_TRY(ar.upload(&d_order, order.data(), order.size(), stream));
     PGX_TRY(ar.zeros(&d_bpack, std::max<size_t>(ntot, 1), stream));
@@ -3196,11 +3227,14 @@ struct Systems : SystemsBase {
     PGX_TRY(ar.alloc(&d_bptr, count));
     PGX_TRY(ar.alloc(&d_xptr, count));
     PGX_TRY(ar.zeros(&d_next, 1, stream));
+    PGX_TRY(ar.zeros(&d_err, 1, stream));
     PGX_TRY(ar.zeros(&d_res, count, stream));
     PGX_TRY(ar.alloc(&d_desc, count));
     PGX_CUDA(cudaMallocHost(&h_bpack, sizeof(double) * std::max<size_t>(ntot, 1)));
     PGX_CUDA(cudaMallocHost(&h_xpack, sizeof(double) * std::max<size_t>(ntot, 1)));
     PGX_CUDA(cudaMallocHost(&h_res, sizeof(SysResult) * count));
+    PGX_CUDA(cudaMallocHost(&h_err, sizeof(int)));
+    *h_err = 0;
     PGX_CUDA(cudaMallocHost(&h_bptr, sizeof(double*) * count));
     PGX_CUDA(cudaMallocHost(&h_xptr, sizeof(double*) * count));
     h_bptr_cur.assign(count, nullptr);
@@ -3311,8 +3345,14 @@ struct Systems : SystemsBase {
     // the rest of the SM's shared memory, split over its CTAs, holds the
     // triangular solves' vector for every block that fits
     size_t smem = 0;
+    int most = 0;
+    cudaFuncAttributes fa;
+    PGX_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    PGX_CUDA(cudaFuncGetAttributes(&fa, kern));
+    PGX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
     PGX_CUDA(cudaOccupancyAvailableDynamicSMemPerBlock(&smem, kern, cps, th));
-    smem = smem / 256 * 256;
+    // no more than a flow pass uses: the rest stays with the L1 cache
+    smem = std::min(smem / 256 * 256, (SysFlowCfg<P>::bytes + 255) / 256 * 256);
     PGX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (!ord) {
       ord = d_order;
@@ -3333,11 +3373,14 @@ struct Systems : SystemsBase {
     a.lanes = ln;
     a.scap = (int)(smem / sizeof(P));
     a.depth = dp;
+    a.flow = th >= SysFlowCfg<P>::threads && smem >= SysFlowCfg<P>::bytes;
+    a.err = d_err;
     a.next = d_next;
     a.st = d_st;
     a.st_in = d_st_in;
     a.res = d_res;
     PGX_CUDA(cudaMemsetAsync(d_next, 0, sizeof(unsigned int), stream));
+    PGX_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
     PGX_CUDA(cudaEventRecord(ev0, stream));
     kern<<<grid, th, smem, stream>>>(a);
     PGX_CUDA(cudaGetLastError());
@@ -3380,6 +3423,7 @@ struct Systems : SystemsBase {
     }
     PGX_TRY(launch(kdim, maxits, tol, atol, threads, ctas_per_sm, lanes, depth));
     PGX_CUDA(cudaMemcpyAsync(h_res, d_res, sizeof(SysResult) * count, cudaMemcpyDeviceToHost, stream));
+    PGX_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     if (location == PGX_LOCATION_HOST)
       PGX_CUDA(cudaMemcpyAsync(h_xpack, d_xpack, sizeof(double) * ntot, cudaMemcpyDeviceToHost, stream));
     PGX_CUDA(cudaStreamSynchronize(stream));
@@ -3398,7 +3442,10 @@ struct Systems : SystemsBase {
       t_end[s] = (double)(r.t1 - tmin) * 1e-6;
       t_tri[s] = (double)r.tri_ns * 1e-6;
       int st = PGX_SUCCESS;
-      if (!std::isfinite(r.normr) || !std::isfinite(r.true_r2)) {
+      if (*h_err) {
+        st = PGX_ERROR_TIMEOUT;
+        if (out == PGX_SUCCESS) out = fail(st, "triangular-solve staging wait timed out");
+      } else if (!std::isfinite(r.normr) || !std::isfinite(r.true_r2)) {
         st = PGX_ERROR_NOT_FINITE;
         if (out == PGX_SUCCESS) out = fail(st, "system %d: FGMRES residual is not finite", s);
       }

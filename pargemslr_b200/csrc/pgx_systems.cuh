@@ -26,6 +26,7 @@
 #pragma once
 
 #include "pgx_device.cuh"
+#include "pgx_flow.cuh"
 
 namespace pgx {
 
@@ -66,6 +67,12 @@ struct SysTri {
   const P* hva;
   const int* dst;
   const P* dinv;
+  // the same factor as task images (SysFlowCfg layout); no chunks: the
+  // packed rows above are used
+  int nchunks;
+  const int* chunk;
+  const int* first;
+  const unsigned char* blob;
 };
 
 template <typename P>
@@ -124,6 +131,8 @@ struct SysArgs {
   int lanes;          // SpMV lanes per row (1, 2, 4 or 8)
   int scap;           // values of the dynamic shared-memory solve buffer
   int depth;          // levels the triangular passes fetch ahead (2 or 3)
+  int flow;           // the CTA's threads and shared memory hold a flow pass
+  int* err;
   unsigned int* next;
   FgmresDev* st;      // per CTA: outer solve
   FgmresDev* st_in;   // per CTA: inner solve
@@ -132,7 +141,11 @@ struct SysArgs {
 
 // shared memory of one CTA: reduction partials, coefficient vectors and the
 // products an update applies
+template <typename P>
 struct SysShared {
+  FlowShared<SysFlowCfg<P>> flow;
+  int use_flow;
+  int* err;
   double red[kSysDotCols * 32];
   void* sbuf;  // the CTA's triangular-solve buffer (dynamic shared memory)
   int scap;    // its capacity in values
@@ -203,9 +216,9 @@ __device__ void sys_multidot(int n, int ncols, const TV* V, long long ld, const 
 // zero); returns the block sum of out(i)^2 when NORM.  coef may live in
 // global or shared memory; the products sign * msc[c] * coef[c] are formed
 // once in shared memory.
-template <bool NORM, typename TM, typename TI, typename TO>
+template <bool NORM, typename P, typename TM, typename TI, typename TO>
 __device__ double sys_update(int n, int ncols, const TM* M, long long ld, const double* msc, const double* coef,
-                             double sign, const TI* in, double isc, TO* out, SysShared& sh) {
+                             double sign, const TI* in, double isc, TO* out, SysShared<P>& sh) {
   for (int c = threadIdx.x; c < ncols; c += blockDim.x) sh.prod[c] = sign * (msc ? msc[c] : 1.0) * coef[c];
   __syncthreads();
   double nrm[1] = {0.0};
@@ -345,73 +358,103 @@ __device__ __noinline__ void sys_trsv(const SysTri<P>& T, const P* rhs, P* out, 
   }
 }
 
-// x = U^-1 L^-1 rhs of level l (GemslrClass::SolveB): rhs is gathered into
-// the lower factor's packed order, the lower pass writes its result in the
-// upper factor's packed order and the upper pass writes x in row order.
-// Each pass keeps its solved values in the CTA's shared ring when the
-// factor's span fits (ring = the largest power of two within the shared
-// buffer), else in the system's packed scratch vector.
+// One pass by dataflow (pgx_flow.cuh), the whole level as one subdomain.  The
+// chain of dependency levels bounds it, at about 0.15 us a level where the
+// barrier-a-level pass below takes 0.7: 40 systems of 32^2 to 112^2, mixed, in
+// one launch on a B200, 52 ms against 175 ms.
+template <bool UPPER, int MAXT, typename P>
+__device__ __noinline__ void sys_flow(const SysTri<P>& T, const P* yu, const P* rhs, P* x, SysShared<P>& sh) {
+  FlowArgs a;
+  a.n = T.n;
+  a.chunk = (const int4*)T.chunk;
+  a.comp_chunk0 = nullptr;
+  a.first = (const int2*)T.first;
+  a.blob = T.blob;
+  PtrR<P, 1> py, pr, px;
+  py.p[0] = const_cast<P*>(yu);
+  pr.p[0] = const_cast<P*>(rhs);
+  px.p[0] = x;
+  flow_pass<P, UPPER, 1, SysFlowCfg<P>>(sh.flow, (unsigned char*)sh.sbuf, a, 0, 0, T.nchunks, py, pr, px, sh.err);
+  __syncthreads();
+  flow_end(sh.flow);
+}
+
+// x = U^-1 L^-1 rhs of level l (GemslrClass::SolveB): the lower pass writes
+// its result in the upper factor's packed order and the upper pass writes x
+// in row order.  A factor laid out as task images runs by dataflow; for the
+// others the lower pass's rhs is gathered into its packed order, and the pass
+// keeps its solved values in the CTA's shared ring when the factor's span
+// fits (ring = the largest power of two within the shared buffer), else in
+// the system's packed scratch vector.
 template <int MAXT, typename P>
-__device__ void sys_solve_b(const SysDesc<P>& d, int l, const P* rhs, P* x, P* sbuf, int scap, int depth,
-                            unsigned long long* tri_ns) {
+__device__ void sys_solve_b(const SysDesc<P>& d, int l, const P* rhs, P* x, SysShared<P>& sh) {
   const unsigned long long t0 = threadIdx.x == 0 ? sys_clock() : 0ull;
+  P* const sbuf = (P*)sh.sbuf;
+  const int scap = sh.scap;
   const SysLevel<P>& v = d.lev[l];
   const unsigned ring = scap > 0 ? 1u << (31 - __clz(scap)) : 0u;
   const bool lr = v.L.span < (int)ring, ur = v.U.span < (int)ring;
-  constexpr int G = 4;  // gathers in flight per thread
-  for (int k0 = threadIdx.x; k0 < v.nl; k0 += G * blockDim.x) {
-    int r[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) r[g] = k0 + g * (int)blockDim.x < v.nl ? v.L.row[k0 + g * blockDim.x] : -1;
-    P q[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) q[g] = r[g] >= 0 ? rhs[r[g]] : P(0);
-#pragma unroll
-    for (int g = 0; g < G; g++)
-      if (r[g] >= 0) d.yr[k0 + g * blockDim.x] = q[g];
-  }
-  __syncthreads();
-  if (depth == 3) {
-    sys_trsv<false, 3, MAXT>(v.L, (const P*)d.yr, d.yu, lr ? sbuf : d.y, lr ? ring - 1 : 0xFFFFFFFFu);
-    sys_trsv<true, 3, MAXT>(v.U, (const P*)d.yu, x, ur ? sbuf : d.y, ur ? ring - 1 : 0xFFFFFFFFu);
+  if (sh.use_flow && v.L.nchunks > 0) {
+    sys_flow<false, MAXT>(v.L, (const P*)d.yu, rhs, (P*)nullptr, sh);
   } else {
-    sys_trsv<false, 2, MAXT>(v.L, (const P*)d.yr, d.yu, lr ? sbuf : d.y, lr ? ring - 1 : 0xFFFFFFFFu);
-    sys_trsv<true, 2, MAXT>(v.U, (const P*)d.yu, x, ur ? sbuf : d.y, ur ? ring - 1 : 0xFFFFFFFFu);
+    constexpr int G = 4;  // gathers in flight per thread
+    for (int k0 = threadIdx.x; k0 < v.nl; k0 += G * blockDim.x) {
+      int r[G];
+#pragma unroll
+      for (int g = 0; g < G; g++) r[g] = k0 + g * (int)blockDim.x < v.nl ? v.L.row[k0 + g * blockDim.x] : -1;
+      P q[G];
+#pragma unroll
+      for (int g = 0; g < G; g++) q[g] = r[g] >= 0 ? rhs[r[g]] : P(0);
+#pragma unroll
+      for (int g = 0; g < G; g++)
+        if (r[g] >= 0) d.yr[k0 + g * blockDim.x] = q[g];
+    }
+    __syncthreads();
+    if (sh.depth == 3)
+      sys_trsv<false, 3, MAXT>(v.L, (const P*)d.yr, d.yu, lr ? sbuf : d.y, lr ? ring - 1 : 0xFFFFFFFFu);
+    else
+      sys_trsv<false, 2, MAXT>(v.L, (const P*)d.yr, d.yu, lr ? sbuf : d.y, lr ? ring - 1 : 0xFFFFFFFFu);
   }
-  if (threadIdx.x == 0) *tri_ns += sys_clock() - t0;
+  if (sh.use_flow && v.U.nchunks > 0)
+    sys_flow<true, MAXT>(v.U, (const P*)d.yu, (const P*)nullptr, x, sh);
+  else if (sh.depth == 3)
+    sys_trsv<true, 3, MAXT>(v.U, (const P*)d.yu, x, ur ? sbuf : d.y, ur ? ring - 1 : 0xFFFFFFFFu);
+  else
+    sys_trsv<true, 2, MAXT>(v.U, (const P*)d.yu, x, ur ? sbuf : d.y, ur ? ring - 1 : 0xFFFFFFFFu);
+  if (threadIdx.x == 0) sh.tri_ns += sys_clock() - t0;
 }
 
 // x += WH (W^T x) in place (SolveApplyLowRankLevel, gemslr.cpp:3585-3590)
 template <typename P>
-__device__ void sys_lowrank(const SysLevel<P>& v, P* x, SysShared& sh) {
+__device__ void sys_lowrank(const SysLevel<P>& v, P* x, SysShared<P>& sh) {
   sys_multidot(v.m, v.rank, v.W, v.m, (const double*)nullptr, x, 1.0, sh.red, sh.coef);
-  sys_update<false>(v.m, v.rank, v.WH, v.m, (const double*)nullptr, sh.coef, 1.0, x, 1.0, x, sh);
+  sys_update<false, P>(v.m, v.rank, v.WH, v.m, (const double*)nullptr, sh.coef, 1.0, x, 1.0, x, sh);
 }
 
 // Orthogonalise column j+1 of the basis against columns 0..j by CGS2, then
 // finish the Hessenberg column with the Givens rotations (one thread).
-template <typename TV>
-__device__ void sys_arnoldi(TV* Vb, long long ld, int j, FgmresDev* st, int nrows, SysShared& sh) {
+template <typename P, typename TV>
+__device__ void sys_arnoldi(TV* Vb, long long ld, int j, FgmresDev* st, int nrows, SysShared<P>& sh) {
   TV* w = Vb + (long long)(j + 1) * ld;
   sys_multidot(nrows, j + 1, Vb, ld, st->sc, w, 1.0, sh.red, sh.coef);
   for (int c = threadIdx.x; c <= j; c += blockDim.x) {
     st->hcol[c] = sh.coef[c];
     st->coefA[c] = sh.coef[c];
   }
-  sys_update<false>(nrows, j + 1, Vb, ld, st->sc, sh.coef, -1.0, w, 1.0, w, sh);
+  sys_update<false, P>(nrows, j + 1, Vb, ld, st->sc, sh.coef, -1.0, w, 1.0, w, sh);
   sys_multidot(nrows, j + 1, Vb, ld, st->sc, w, 1.0, sh.red, sh.coef2);
   for (int c = threadIdx.x; c <= j; c += blockDim.x) {
     st->hcol[c] += sh.coef2[c];
     st->coefB[c] = sh.coef2[c];
   }
-  const double t2 = sys_update<true>(nrows, j + 1, Vb, ld, st->sc, sh.coef2, -1.0, w, 1.0, w, sh);
+  const double t2 = sys_update<true, P>(nrows, j + 1, Vb, ld, st->sc, sh.coef2, -1.0, w, 1.0, w, sh);
   __syncthreads();
   if (threadIdx.x == 0) fgmres_givens(st, j, sqrt(t2));
   __syncthreads();
 }
 
 template <int MAXT, typename P>
-__device__ void sys_inner_solve(const SysDesc<P>& d, P* xl, const P* zl, FgmresDev* st, int S, SysShared& sh);
+__device__ void sys_inner_solve(const SysDesc<P>& d, P* xl, const P* zl, FgmresDev* st, int S, SysShared<P>& sh);
 
 // GemslrClass::SolveLevel from level l0 down (gemslr.cpp:3474-3630) with the
 // recursion unrolled: the descent keeps each level's right-hand side, the
@@ -420,7 +463,7 @@ __device__ void sys_inner_solve(const SysDesc<P>& d, P* xl, const P* zl, FgmresD
 // in place of the low-rank correction and the lower levels.
 template <bool INNER, int MAXT, typename P>
 __device__ void sys_solve_from(const SysDesc<P>& d, int l0, P* x, const P* rhs, FgmresDev* st_in, int S,
-                               SysShared& sh) {
+                               SysShared<P>& sh) {
   const P* rh[kSysMaxLevels];
   P* xs[kSysMaxLevels];
   int l = l0;
@@ -437,7 +480,7 @@ __device__ void sys_solve_from(const SysDesc<P>& d, int l0, P* x, const P* rhs, 
       for (int i = threadIdx.x; i < v.m; i += blockDim.x) zl[i] = r[v.nl + i];
       __syncthreads();
     } else {
-      sys_solve_b<MAXT>(d, l, r, zu, (P*)sh.sbuf, sh.scap, sh.depth, &sh.tri_ns);  // 1. zu = B^-1 rhs_u
+      sys_solve_b<MAXT>(d, l, r, zu, sh);  // 1. zu = B^-1 rhs_u
       sys_spmv<P>(v.E, (const P*)zu, P(-1), r + v.nl, P(1), zl, S);   // 2-3. zl = rhs_l - E zu
     }
     if (INNER && l == 0 && d.inner) {
@@ -453,14 +496,14 @@ __device__ void sys_solve_from(const SysDesc<P>& d, int l0, P* x, const P* rhs, 
   if (stop_inner) {
     top = l;
   } else {
-    sys_solve_b<MAXT>(d, d.nlev - 1, r, xv, (P*)sh.sbuf, sh.scap, sh.depth, &sh.tri_ns);  // last level
+    sys_solve_b<MAXT>(d, d.nlev - 1, r, xv, sh);  // last level
     top = d.nlev - 2;
   }
   for (int t = top; t >= l0; t--) {
     const SysLevel<P>& v = d.lev[t];
     P* zu = v.z;
     sys_spmv<P>(v.F, (const P*)(xs[t] + v.nl), P(-1), rh[t], P(1), zu, S);  // 5-6. zu = rhs_u - F xl
-    sys_solve_b<MAXT>(d, t, zu, xs[t], (P*)sh.sbuf, sh.scap, sh.depth, &sh.tri_ns);  // 7. xu = B^-1 zu
+    sys_solve_b<MAXT>(d, t, zu, xs[t], sh);  // 7. xu = B^-1 zu
   }
 }
 
@@ -469,7 +512,7 @@ __device__ void sys_solve_from(const SysDesc<P>& d, int l0, P* x, const P* rhs, 
 // is the low-rank correction followed by the level-1 recursion
 // (GemslrSchurMatrixClass::Solve, gemslr.cpp:294-330).
 template <int MAXT, typename P>
-__device__ void sys_inner_solve(const SysDesc<P>& d, P* xl, const P* zl, FgmresDev* st, int S, SysShared& sh) {
+__device__ void sys_inner_solve(const SysDesc<P>& d, P* xl, const P* zl, FgmresDev* st, int S, SysShared<P>& sh) {
   const SysLevel<P>& v0 = d.lev[0];
   const int m0 = v0.m;
   const long long ld = m0;
@@ -509,23 +552,23 @@ __device__ void sys_inner_solve(const SysDesc<P>& d, P* xl, const P* zl, FgmresD
     P* wj = d.Vin + (long long)(j + 1) * ld;
     const double scj = st->sc[j];
     if (v0.rank > 0) sys_multidot(m0, v0.rank, v0.W, ld, (const double*)nullptr, vj, scj, sh.red, sh.coef);
-    sys_update<false>(m0, v0.rank, v0.WH, ld, (const double*)nullptr, sh.coef, 1.0, vj, scj, d.xlr, sh);
+    sys_update<false, P>(m0, v0.rank, v0.WH, ld, (const double*)nullptr, sh.coef, 1.0, vj, scj, d.xlr, sh);
     sys_solve_from<false, MAXT>(d, 1, zj, (const P*)d.xlr, st, S, sh);
     // w = S0 z (GemslrClass::SchurMatVec, gemslr.cpp:3799-3960)
     sys_spmv<P>(v0.F, (const P*)zj, P(1), (const P*)nullptr, P(0), d.s_zu, S);
-    sys_solve_b<MAXT>(d, 0, d.s_zu, d.s_wu, (P*)sh.sbuf, sh.scap, sh.depth, &sh.tri_ns);
+    sys_solve_b<MAXT>(d, 0, d.s_zu, d.s_wu, sh);
     sys_spmv<P>(d.C0, (const P*)zj, P(1), (const P*)nullptr, P(0), wj, S);
     sys_spmv<P>(v0.E, (const P*)d.s_wu, P(-1), (const P*)wj, P(1), wj, S);
     sys_arnoldi(d.Vin, ld, j, st, m0, sh);
   }
   const int ni = *(volatile int*)&st->i;
-  sys_update<false>(m0, ni, d.Zin, ld, (const double*)nullptr, st->rs, 1.0, (const P*)nullptr, 1.0, xl, sh);
+  sys_update<false, P>(m0, ni, d.Zin, ld, (const double*)nullptr, st->rs, 1.0, (const P*)nullptr, 1.0, xl, sh);
 }
 
 // GemslrClass::Solve (gemslr.cpp:3431-3472): z = Q^T M^-1 P v with v scaled
 template <int MAXT, typename P>
 __device__ void sys_precond(const SysDesc<P>& d, const double* v, double vsc, P* z, FgmresDev* st_in, int S,
-                            SysShared& sh) {
+                            SysShared<P>& sh) {
   for (int i = threadIdx.x; i < d.n; i += blockDim.x) d.rt[i] = (P)(v[d.pperm[i]] * vsc);
   __syncthreads();
   sys_solve_from<true, MAXT>(d, 0, d.xt, (const P*)d.rt, st_in, S, sh);
@@ -539,12 +582,14 @@ __device__ void sys_precond(const SysDesc<P>& d, const double* v, double vsc, P*
 // autotuner tries both).
 template <typename P, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) systems_fgmres_kernel(SysArgs<P> a) {
-  __shared__ SysShared sh;
+  __shared__ __align__(16) SysShared<P> sh;
   extern __shared__ __align__(16) unsigned char sys_dyn[];
   if (threadIdx.x == 0) {
     sh.sbuf = sys_dyn;
     sh.scap = a.scap;
     sh.depth = a.depth;
+    sh.use_flow = a.flow;
+    sh.err = a.err;
   }
   __syncthreads();
   FgmresDev* st = a.st + blockIdx.x;
@@ -633,7 +678,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) systems_fgmres_kern
       }
       // x += Z y  (fgmres.hpp:471-490)
       const int ni = *(volatile int*)&st->i;
-      sys_update<false>(n, ni, d.Z, ld, (const double*)nullptr, st->rs, 1.0, (const double*)x, 1.0, x, sh);
+      sys_update<false, P>(n, ni, d.Z, ld, (const double*)nullptr, st->rs, 1.0, (const double*)x, 1.0, x, sh);
       if (!*(volatile int*)&st->done)
         sys_spmv<double>(d.A, (const double*)x, -1.0, b, 1.0, d.V, S);                 // restart residual
       if (threadIdx.x == 0) {
