@@ -807,7 +807,6 @@ template <typename P>
 struct Engine;
 template <typename P>
 int make_batch_slot(Engine<P>& own, Import& im, int lanes, std::unique_ptr<EngineBase>& out);
-constexpr int kMaxLanes = 16;  // right-hand sides one slot advances together
 
 template <typename P>
 struct Engine : EngineBase {
@@ -997,7 +996,7 @@ struct Engine : EngineBase {
           if (rc != PGX_SUCCESS && rc != PGX_ERROR_INVALID_PARAM) return rc;
       }
       if (rcL == PGX_SUCCESS && rcU == PGX_SUCCESS) {
-        // one CTA per subdomain; y travels from the lower to the upper pass in slot order
+        // one product, or one CTA per subdomain (y travels from the lower to the upper pass in slot order)
       } else if (use_seg && want_segments(h.L, SegCfg<P>::nnz) && want_segments(h.U, SegCfg<P>::nnz)) {
         d.L = DTri<P>();
         d.U = DTri<P>();
@@ -2223,6 +2222,8 @@ struct BatchEngine : EngineBase {
   cudaStream_t stream = nullptr;
   Arena wk;
   std::vector<std::array<P*, R>> yslot;  // per level, in the R-layout's slot order
+  using F = typename Engine<P>::F;
+  using SD = typename Engine<P>::SD;
   int n = 0, nlev = 0;
   // Block low-rank correction on the tensor cores: complex64 slots of 8 or
   // 16 lanes apply W^H X and X + WH Y to all lanes in two tcgen05 GEMMs
@@ -2420,6 +2421,120 @@ struct BatchEngine : EngineBase {
     trsv_b(l, true, none, y, x, sk);
   }
 
+  // one launch of a tall-skinny kernel for every lane
+  template <typename TV, typename TM, typename TW, int MODE>
+  void ts_b(const std::array<TsArgs<TV, TM, TW>, R>& a) {
+    TsLanes<TV, TM, TW> p;
+    for (int r = 0; r < R; r++) {
+      p.a[r] = a[r];
+      p.a[r].partial = lane[r]->partial;
+      p.a[r].counter = lane[r]->counter;
+    }
+    const dim3 grid(grid_for(a[0].n, kTsThreads, kTsMaxBlocks), R);
+    ts_lanes_kernel<TV, TM, TW, MODE><<<grid, kTsThreads, 0, stream>>>(p);
+  }
+  // Engine::spmv for every lane
+  template <typename TA, typename TX, typename TY, typename TC, typename X1, typename X2, typename B, typename Y>
+  void spmv_b(const DCsr<TA>& M, const X1& x, TC alpha, const DCsr<TA>* M2, const X2* x2, TC alpha2, const B* b,
+              TC beta, const Y& y, const std::array<Skip, R>& sk) {
+    if (M.rows == 0) return;
+    if (M.merge && !M2) {  // the merge path keeps its carries per lane
+      for (int r = 0; r < R; r++)
+        lane[r]->template spmv<TA, TX, TY, TC>(M, x[r], alpha, nullptr, nullptr, TC(0), b ? (*b)[r] : nullptr, beta,
+                                               y[r], nullptr, sk[r]);
+      return;
+    }
+    SpmvLanes<TX, TY> p;
+    for (int r = 0; r < R; r++) {
+      p.x1[r] = x[r];
+      p.x2[r] = x2 ? (*x2)[r] : nullptr;
+      p.b[r] = b ? (*b)[r] : nullptr;
+      p.y[r] = y[r];
+      p.err[r] = lane[r]->err;
+      p.skip[r] = sk[r];
+    }
+    const dim3 grid(grid_for(M.rows, 256 / M.S, num_sms() * 16), R);
+    const int *rp2 = M2 ? M2->rp : nullptr, *cj2 = M2 ? M2->cj : nullptr;
+    const TA* va2 = M2 ? M2->va : nullptr;
+    const int xcols2 = M2 ? M2->cols : 0;
+#define PGX_SPMVL(SS)                                                                                                 \
+  spmv_lanes_kernel<TA, TX, TY, TC, SS><<<grid, 256, 0, stream>>>(M.rows, M.rp, M.cj, M.va, M.cols, alpha, rp2, cj2, \
+                                                                  va2, xcols2, alpha2, beta, p)
+    switch (M.S) {
+      case 2: PGX_SPMVL(2); break;
+      case 4: PGX_SPMVL(4); break;
+      case 8: PGX_SPMVL(8); break;
+      case 16: PGX_SPMVL(16); break;
+      default: PGX_SPMVL(32); break;
+    }
+#undef PGX_SPMVL
+  }
+  // Engine::arnoldi_step for every lane
+  template <typename TV, typename TW>
+  void arnoldi_b(const std::array<TV*, R>& Vb, long long ld, int j, const std::array<SD*, R>& s, int nrows,
+                 const std::array<Skip, R>& sk) {
+    std::array<TsArgs<TV, TV, TW>, R> a;
+    for (int r = 0; r < R; r++) {
+      a[r] = Engine<P>::template ts_args<TV, TV, TW>(nrows, sk[r]);
+      a[r].ncols = j + 1;
+      a[r].V = Vb[r];
+      a[r].ldv = ld;
+      a[r].vsc = s[r]->sc;
+      a[r].in = (TW*)(Vb[r] + (long long)(j + 1) * ld);
+      a[r].epi = EPI_CGS_FIRST;
+      a[r].st = s[r];
+    }
+    ts_b<TV, TV, TW, TS_DOT>(a);
+    for (int r = 0; r < R; r++) {
+      a[r].M = Vb[r];
+      a[r].ldm = ld;
+      a[r].msc = s[r]->sc;
+      a[r].coef = s[r]->coefA;
+      a[r].sign = -1.0;
+      a[r].out = (TW*)(Vb[r] + (long long)(j + 1) * ld);
+      a[r].epi = EPI_CGS_SECOND;
+    }
+    ts_b<TV, TV, TW, TS_UPDATE_DOT>(a);
+    for (int r = 0; r < R; r++) {
+      a[r].coef = s[r]->coefB;
+      a[r].epi = EPI_GIVENS;
+      a[r].j = j;
+    }
+    ts_b<TV, TV, TW, TS_UPDATE_NORM>(a);
+  }
+  // out = v s + WH (W^H (v s)) at level l for every lane (s: the lane's scale, or none)
+  void lowrank_b(int l, const std::array<const P*, R>& v, const std::array<const double*, R>& scale,
+                 const std::array<P*, R>& out, const std::array<Skip, R>& sk) {
+    const int rank = lane[0]->lv[l].rank, m = lane[0]->lv[l].m;
+    std::array<TsArgs<P, P, P>, R> a;
+    if (rank > 0) {
+      for (int r = 0; r < R; r++) {
+        DLevel<P>& d = lane[r]->lv[l];
+        a[r] = Engine<P>::template ts_args<P, P, P>(m, sk[r]);
+        a[r].ncols = rank;
+        a[r].V = d.W;
+        a[r].ldv = m;
+        a[r].in = v[r];
+        a[r].in_scale = scale[r];
+        a[r].epi = EPI_STORE;
+        a[r].dst = d.lrt;
+      }
+      ts_b<P, P, P, TS_DOT>(a);
+    }
+    for (int r = 0; r < R; r++) {
+      DLevel<P>& d = lane[r]->lv[l];
+      a[r] = Engine<P>::template ts_args<P, P, P>(m, sk[r]);
+      a[r].ncols = rank;
+      a[r].M = d.WH;
+      a[r].ldm = m;
+      a[r].coef = d.lrt;
+      a[r].in = v[r];
+      a[r].in_scale = scale[r];
+      a[r].out = out[r];
+    }
+    ts_b<P, P, P, TS_UPDATE>(a);
+  }
+
   // Engine::solve_level for every lane
   void solve_level_b(int l, const std::array<P*, R>& x, const std::array<const P*, R>& rhs,
                      const std::array<Skip, R>& sk) {
@@ -2427,185 +2542,172 @@ struct BatchEngine : EngineBase {
       solve_b_b(l, rhs, x, sk);
       return;
     }
-    const int nl = lane[0]->lv[l].nl;
+    const DLevel<P>& d0 = lane[0]->lv[l];
+    const int nl = d0.nl;
     std::array<P*, R> zu, zl, xl;
-    std::array<const P*, R> czu, czl;
+    std::array<const P*, R> czu, czl, rhs_l;
     for (int r = 0; r < R; r++) {
       zu[r] = lane[r]->lv[l].z;
       zl[r] = zu[r] + nl;
       xl[r] = x[r] + nl;
       czu[r] = zu[r];
       czl[r] = zl[r];
+      rhs_l[r] = rhs[r] + nl;
     }
     if (lane[0]->usolve) {  // U solve: zl = rhs_l
+      PermLanes<P, P> p;
       for (int r = 0; r < R; r++) {
-        const int m = lane[r]->lv[l].m;
-        gather_kernel<P, P><<<grid_for(m, 256 * kPermUnroll, num_sms() * 16), 256, 0, stream>>>(
-            m, nullptr, rhs[r] + nl, nullptr, zl[r], sk[r]);
+        p.in[r] = rhs_l[r];
+        p.scale[r] = nullptr;
+        p.out[r] = zl[r];
+        p.skip[r] = sk[r];
       }
+      gather_lanes_kernel<P, P><<<dim3(grid_for(d0.m, 256 * kPermUnroll, num_sms() * 16), R), 256, 0, stream>>>(
+          d0.m, nullptr, p);
     } else {
       solve_b_b(l, rhs, zu, sk);
-      for (int r = 0; r < R; r++) {
-        DLevel<P>& d = lane[r]->lv[l];
-        lane[r]->template spmv<P, P, P, P>(d.E, zu[r], (P)-1, nullptr, nullptr, (P)0, rhs[r] + nl, (P)1, zl[r],
-                                           nullptr, sk[r]);
-      }
+      spmv_b<P, P, P, P>(d0.E, zu, (P)-1, nullptr, (const std::array<P*, R>*)nullptr, (P)0, &rhs_l, (P)1, zl, sk);
     }
     if (l == 0 && lane[0]->inner) {
       inner_solve_b(xl, czl, sk);
     } else {
-      if (use_lowrank_block(l)) {
-        std::array<const P*, R> czl2;
-        std::array<const double*, R> none;
-        for (int r = 0; r < R; r++) {
-          czl2[r] = zl[r];
-          none[r] = nullptr;
-        }
-        lowrank_block(l, czl2, zl, none, sk);
-      } else {
-        for (int r = 0; r < R; r++)
-          if (lane[r]->lv[l].rank > 0) lane[r]->lowrank_inplace(l, zl[r], sk[r]);
-      }
+      std::array<const double*, R> none;
+      none.fill(nullptr);
+      if (use_lowrank_block(l))
+        lowrank_block(l, czl, zl, none, sk);
+      else if (d0.rank > 0)
+        lowrank_b(l, czl, none, zl, sk);
       solve_level_b(l + 1, xl, czl, sk);
     }
-    for (int r = 0; r < R; r++) {
-      DLevel<P>& d = lane[r]->lv[l];
-      lane[r]->template spmv<P, P, P, P>(d.F, xl[r], (P)-1, nullptr, nullptr, (P)0, rhs[r], (P)1, zu[r], nullptr,
-                                         sk[r]);
-    }
+    spmv_b<P, P, P, P>(d0.F, xl, (P)-1, nullptr, (const std::array<P*, R>*)nullptr, (P)0, &rhs, (P)1, zu, sk);
     solve_b_b(l, czu, x, sk);
   }
 
   // Engine::inner_solve for every lane
   void inner_solve_b(const std::array<P*, R>& xl, const std::array<const P*, R>& zl,
                      const std::array<Skip, R>& outer) {
-    const int m0 = lane[0]->lv[0].m;
+    const DLevel<P>& d0 = lane[0]->lv[0];
+    const int m0 = d0.m;
     const long long ld = m0;
     const int kin = lane[0]->inner_maxits;
+    std::array<TsArgs<P, P, P>, R> a;
+    std::array<P*, R> Vin, xlr, szu, swu;
+    std::array<const P*, R> cxlr, cszu;
+    std::array<SD*, R> st_in;
+    std::array<Skip, R> it;
     for (int r = 0; r < R; r++) {
       Engine<P>& e = *lane[r];
-      auto a = Engine<P>::template ts_args<P, P, P>(m0, outer[r]);
-      a.in = zl[r];
-      a.out = e.Vin;
-      a.epi = EPI_INIT_INNER;
-      a.st = e.st_in;
-      e.template ts<P, P, P, TS_NORM_COPY>(a);
+      a[r] = Engine<P>::template ts_args<P, P, P>(m0, outer[r]);
+      a[r].in = zl[r];
+      a[r].out = e.Vin;
+      a[r].epi = EPI_INIT_INNER;
+      a[r].st = e.st_in;
+      Vin[r] = e.Vin;
+      st_in[r] = e.st_in;
+      xlr[r] = e.lv[0].xlr;
+      cxlr[r] = xlr[r];
+      szu[r] = e.s_zu;
+      swu[r] = e.s_wu;
+      cszu[r] = e.s_zu;
+      it[r] = mk_skip(outer[r].f0, outer[r].f1, &e.st_in->cycle_done);
     }
+    ts_b<P, P, P, TS_NORM_COPY>(a);
     for (int j = 0; j < kin; j++) {
-      std::array<Skip, R> it;
-      std::array<P*, R> zj, xlr, szu, swu;
-      std::array<const P*, R> cxlr, cszu;
-      const bool block = use_lowrank_block(0);
-      std::array<const P*, R> vjs;
-      std::array<const double*, R> scs;
+      std::array<P*, R> zj, wj;
+      std::array<const P*, R> vj;
+      std::array<const double*, R> sc;
       for (int r = 0; r < R; r++) {
         Engine<P>& e = *lane[r];
-        DLevel<P>& d0 = e.lv[0];
-        it[r] = mk_skip(outer[r].f0, outer[r].f1, &e.st_in->cycle_done);
-        P* vj = e.Vin + (long long)j * ld;
+        vj[r] = e.Vin + (long long)j * ld;
+        wj[r] = e.Vin + (long long)(j + 1) * ld;
         zj[r] = e.Zin + (long long)j * ld;
-        vjs[r] = vj;
-        scs[r] = &e.st_in->sc[j];
-        if (block) {
-          // xlr = v + WH W^H v for all lanes below
-        } else if (d0.rank > 0) {
-          auto a = Engine<P>::template ts_args<P, P, P>(m0, it[r]);
-          a.ncols = d0.rank;
-          a.V = d0.W;
-          a.ldv = m0;
-          a.in = vj;
-          a.in_scale = &e.st_in->sc[j];
-          a.epi = EPI_STORE;
-          a.dst = d0.lrt;
-          e.template ts<P, P, P, TS_DOT>(a);
-        }
-        if (!block) {
-          auto u = Engine<P>::template ts_args<P, P, P>(m0, it[r]);
-          u.ncols = d0.rank;
-          u.M = d0.WH;
-          u.ldm = m0;
-          u.coef = d0.lrt;
-          u.in = vj;
-          u.in_scale = &e.st_in->sc[j];
-          u.out = d0.xlr;
-          e.template ts<P, P, P, TS_UPDATE>(u);
-        }
-        xlr[r] = d0.xlr;
-        cxlr[r] = d0.xlr;
-        szu[r] = e.s_zu;
-        swu[r] = e.s_wu;
-        cszu[r] = e.s_zu;
+        sc[r] = &e.st_in->sc[j];
       }
-      if (block) lowrank_block(0, vjs, xlr, scs, it);
+      if (use_lowrank_block(0))
+        lowrank_block(0, vj, xlr, sc, it);
+      else
+        lowrank_b(0, vj, sc, xlr, it);
       solve_level_b(1, zj, cxlr, it);
-      for (int r = 0; r < R; r++) {
-        Engine<P>& e = *lane[r];
-        e.template spmv<P, P, P, P>(e.lv[0].F, zj[r], (P)1, nullptr, nullptr, (P)0, (const P*)nullptr, (P)0, szu[r],
-                                    nullptr, it[r]);
-      }
+      spmv_b<P, P, P, P>(d0.F, zj, (P)1, nullptr, (const std::array<P*, R>*)nullptr, (P)0,
+                         (const std::array<const P*, R>*)nullptr, (P)0, szu, it);
       solve_b_b(0, cszu, swu, it);
-      for (int r = 0; r < R; r++) {
-        Engine<P>& e = *lane[r];
-        P* wj = e.Vin + (long long)(j + 1) * ld;
-        e.template spmv<P, P, P, P>(e.C0, zj[r], (P)1, &e.lv[0].E, swu[r], (P)-1, (const P*)nullptr, (P)0, wj,
-                                    nullptr, it[r]);
-        e.template arnoldi_step<P, P>(e.Vin, ld, j, e.st_in, m0, it[r]);
-      }
+      spmv_b<P, P, P, P>(lane[0]->C0, zj, (P)1, &d0.E, &swu, (P)-1, (const std::array<const P*, R>*)nullptr, (P)0, wj,
+                         it);
+      arnoldi_b<P, P>(Vin, ld, j, st_in, m0, it);
     }
     for (int r = 0; r < R; r++) {
       Engine<P>& e = *lane[r];
-      auto u = Engine<P>::template ts_args<P, P, P>(m0, outer[r]);
-      u.ncols_dev = &e.st_in->i;
-      u.M = e.Zin;
-      u.ldm = ld;
-      u.coef = e.st_in->rs;
-      u.in = nullptr;
-      u.out = xl[r];
-      e.template ts<P, P, P, TS_UPDATE>(u);
+      a[r] = Engine<P>::template ts_args<P, P, P>(m0, outer[r]);
+      a[r].ncols_dev = &e.st_in->i;
+      a[r].M = e.Zin;
+      a[r].ldm = ld;
+      a[r].coef = e.st_in->rs;
+      a[r].in = nullptr;
+      a[r].out = xl[r];
     }
+    ts_b<P, P, P, TS_UPDATE>(a);
   }
 
-  // Engine::enqueue_cycle for every lane, preconditioner applies merged
-  using F = typename Engine<P>::F;
+  // Engine::enqueue_cycle for every lane
   void enqueue_cycle_b(int kdim, const std::array<F*, R>& xd, const std::array<const F*, R>& bd) {
     const long long ld = n;
-    std::array<Skip, R> sk;
-    for (int r = 0; r < R; r++) sk[r] = mk_skip(&lane[r]->st->done, &lane[r]->st->cycle_done);
-    const int grid = grid_for(n, 256 * kPermUnroll, num_sms() * 16);  // gather / scatter
-    for (int j = 0; j < kdim; j++) {
-      std::array<P*, R> xt;
-      std::array<const P*, R> rt;
-      for (int r = 0; r < R; r++) {
-        Engine<P>& e = *lane[r];
-        gather_kernel<F, P><<<grid, 256, 0, stream>>>(n, e.pperm, e.V + (long long)j * ld, &e.st->sc[j], e.rt,
-                                                           sk[r]);
-        xt[r] = e.xt;
-        rt[r] = e.rt;
-      }
-      solve_level_b(0, xt, rt, sk);
-      for (int r = 0; r < R; r++) {
-        Engine<P>& e = *lane[r];
-        P* zj = e.Z + (long long)j * ld;
-        scatter_kernel<P, P><<<grid, 256, 0, stream>>>(n, e.qperm ? e.qperm : e.pperm, e.xt, zj, sk[r]);
-        e.template spmv<F, P, F, F>(e.A, zj, 1.0, nullptr, nullptr, 0.0, (const F*)nullptr, 0.0,
-                                                   e.V + (long long)(j + 1) * ld, nullptr, sk[r]);
-        e.template arnoldi_step<F, F>(e.V, ld, j, e.st, n, sk[r]);
-      }
-    }
+    const Engine<P>& e0 = *lane[0];
+    std::array<Skip, R> sk, not_done;
+    std::array<F*, R> V;
+    std::array<SD*, R> st;
+    std::array<P*, R> xt;
+    std::array<const P*, R> rt;
+    StateLanes<F> states;
     for (int r = 0; r < R; r++) {
       Engine<P>& e = *lane[r];
-      auto u = Engine<P>::template ts_args<P, P, F>(n, mk_skip());
-      u.ncols_dev = &e.st->i;
-      u.M = e.Z;
-      u.ldm = ld;
-      u.coef = e.st->rs;
-      u.in = xd[r];
-      u.out = xd[r];
-      e.template ts<P, P, F, TS_UPDATE>(u);
-      e.template spmv<F, F, F, F>(e.A, xd[r], -1.0, nullptr, nullptr, 0.0, bd[r], 1.0, e.V,
-                                                      nullptr, mk_skip(&e.st->done));
-      fgmres_cycle_reset_kernel<<<1, 1, 0, stream>>>(e.st, mk_skip());
+      sk[r] = mk_skip(&e.st->done, &e.st->cycle_done);
+      not_done[r] = mk_skip(&e.st->done);
+      V[r] = e.V;
+      st[r] = e.st;
+      xt[r] = e.xt;
+      rt[r] = e.rt;
+      states.st[r] = e.st;
     }
+    const dim3 grid(grid_for(n, 256 * kPermUnroll, num_sms() * 16), R);  // gather / scatter
+    for (int j = 0; j < kdim; j++) {
+      PermLanes<F, P> g;
+      PermLanes<P, P> c;
+      std::array<P*, R> zj;
+      std::array<F*, R> wj;
+      for (int r = 0; r < R; r++) {
+        Engine<P>& e = *lane[r];
+        zj[r] = e.Z + (long long)j * ld;
+        wj[r] = e.V + (long long)(j + 1) * ld;
+        g.in[r] = e.V + (long long)j * ld;
+        g.scale[r] = &e.st->sc[j];
+        g.out[r] = e.rt;
+        g.skip[r] = sk[r];
+        c.in[r] = e.xt;
+        c.scale[r] = nullptr;
+        c.out[r] = zj[r];
+        c.skip[r] = sk[r];
+      }
+      gather_lanes_kernel<F, P><<<grid, 256, 0, stream>>>(n, e0.pperm, g);
+      solve_level_b(0, xt, rt, sk);
+      scatter_lanes_kernel<P, P><<<grid, 256, 0, stream>>>(n, e0.qperm ? e0.qperm : e0.pperm, c);
+      spmv_b<F, P, F, F>(e0.A, zj, F(1.0), nullptr, (const std::array<P*, R>*)nullptr, F(0.0),
+                         (const std::array<const F*, R>*)nullptr, F(0.0), wj, sk);
+      arnoldi_b<F, F>(V, ld, j, st, n, sk);
+    }
+    std::array<TsArgs<P, P, F>, R> u;
+    for (int r = 0; r < R; r++) {
+      Engine<P>& e = *lane[r];
+      u[r] = Engine<P>::template ts_args<P, P, F>(n, mk_skip());
+      u[r].ncols_dev = &e.st->i;
+      u[r].M = e.Z;
+      u[r].ldm = ld;
+      u[r].coef = e.st->rs;
+      u[r].in = xd[r];
+      u[r].out = xd[r];
+    }
+    ts_b<P, P, F, TS_UPDATE>(u);
+    spmv_b<F, F, F, F>(e0.A, xd, F(-1.0), nullptr, (const std::array<F*, R>*)nullptr, F(0.0), &bd, F(1.0), V, not_done);
+    fgmres_cycle_reset_lanes_kernel<F><<<1, R, 0, stream>>>(states);
   }
 
   int begin_many(int cnt, double* const* x, const double* const* b, int location, int kdim, int maxits, double tol,

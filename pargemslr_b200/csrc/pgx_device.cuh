@@ -19,6 +19,7 @@ using ::__shfl_xor_sync;  // the real forms beside the complex overload
 
 constexpr int kWarp = 32;
 constexpr int KMAX = 128;          // largest Krylov dimension a handle accepts
+constexpr int kMaxLanes = 16;      // right-hand sides one slot advances together
 constexpr int kTsThreads = 512;    // block size of the tall-skinny kernels
 constexpr int kTsMaxBlocks = 296;  // 2 blocks per SM on a 148-SM B200
 constexpr int kSpinLimit = 1 << 21;  // default bound of the waits in the sync-free triangular solves
@@ -120,6 +121,37 @@ __device__ __forceinline__ T group_reduce(T v, int S, int lane) {
   return v;
 }
 
+// Products and sums whose rounding is spelled out, so that a single-lane
+// kernel and its multi-lane form cannot be contracted differently: a slot's
+// results do not depend on its lane count.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ void mac(float& acc, float v, float w) { acc = fmaf(v, w, acc); }
+__device__ __forceinline__ void mac(double& acc, double v, double w) { acc = fma(v, w, acc); }
+template <typename R>
+__device__ __forceinline__ void mac(cplx<R>& acc, const cplx<R>& v, const cplx<R>& w) {
+  acc.x = fma(v.x, w.x, acc.x);
+  acc.y = fma(v.x, w.y, acc.y);
+  acc.x = fma(-v.y, w.y, acc.x);
+  acc.y = fma(v.y, w.x, acc.y);
+}
+template <typename R>
+__device__ __forceinline__ cplx<R> mul_rn(const cplx<R>& a, const cplx<R>& b) {
+  cplx<R> t(mul_rn(a.x, b.x), mul_rn(a.x, b.y));
+  t.x = fma(-a.y, b.y, t.x);
+  t.y = fma(a.y, b.x, t.y);
+  return t;
+}
+__device__ __forceinline__ cf64 mul_rn(const cf64& a, double s) { return cf64(__dmul_rn(a.x, s), __dmul_rn(a.y, s)); }
+__device__ __forceinline__ double abs2_rn(double v) { return __dmul_rn(v, v); }
+__device__ __forceinline__ double abs2_rn(const cf64& v) { return fma(v.x, v.x, __dmul_rn(v.y, v.y)); }
+
+// lane l's value for the whole warp
+__device__ __forceinline__ double bcast(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ cf64 bcast(const cf64& v, int l) {
+  return cf64(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_reduce(T v) {
 #pragma unroll
@@ -159,11 +191,11 @@ __device__ __forceinline__ TC row_dot(int k1, int k2, int lane, const int* __res
   TC acc = 0;
 #pragma unroll
   for (int u = 0; u < kSpmvUnroll; u++)
-    if (c[u] >= 0) acc += (TC)v[u] * (TC)xv[u];
+    if (c[u] >= 0) mac(acc, (TC)v[u], (TC)xv[u]);
   for (int k = k1 + lane + kSpmvUnroll * S; k < k2; k += S) {
     const int cc = __ldg(&cj[k]);
     if ((unsigned)cc < (unsigned)xcols)
-      acc += (TC)ldg(&va[k]) * (TC)x[cc];
+      mac(acc, (TC)ldg(&va[k]), (TC)x[cc]);
     else
       bad = true;
   }
@@ -237,7 +269,7 @@ __device__ __forceinline__ TC row_dot_vec(int k1, int k2, int lane, const int* _
     for (int u = 0; u < 4; u++) xv[u] = in[u] ? x[c[u]] : TX(0);
 #pragma unroll
     for (int u = 0; u < 4; u++)
-      if (in[u]) acc += (TC)v[u] * (TC)xv[u];
+      if (in[u]) mac(acc, (TC)v[u], (TC)xv[u]);
   }
   return acc;
 }
@@ -267,9 +299,9 @@ __device__ __forceinline__ void spmv_rows(
       acc2 = group_reduce(acc2, S, wlane);
     }
     if (lane == 0) {
-      TC v = alpha * (acc * xs);
-      if (rp2) v += alpha2 * acc2;
-      if (b) v += beta * (TC)b[row];
+      TC v = mul_rn(alpha, mul_rn(acc, xs));
+      if (rp2) mac(v, alpha2, acc2);
+      if (b) mac(v, beta, (TC)b[row]);
       y[row] = (TY)v;
     }
   }
@@ -989,31 +1021,115 @@ __device__ inline void fgmres_givens(FgmresDevT<S>* st, int j, double t) {
   }
 }
 
+// The same by a whole block (the last one of a reduction), for the kernel
+// whose end is on the critical path of every Krylov step: one thread read the
+// state word by word from global memory (ncu, inner steps of a 64^3 solve:
+// 12.4 us a launch then, 10.7 us now; of outer steps 17.0 and 14.2 us).
+// The column, the rotations and the scalars are read by all threads at once,
+// thread 0 rotates in shared memory, and one warp substitutes back with the
+// next column of H on its way.  `sh` holds 3 * (KMAX + 1) values.
+template <typename S>
+__device__ inline void fgmres_givens_block(FgmresDevT<S>* st, int j, double t, S* sh, int* s_back) {
+  const int ldh = KMAX + 1, tid = threadIdx.x;
+  S *h = sh, *rc = sh + ldh, *rs_ = sh + 2 * ldh;
+  for (int c = tid; c <= j; c += blockDim.x) {
+    h[c] = st->hcol[c];
+    if (c < j) {
+      rc[c] = st->c[c];
+      rs_[c] = st->s[c];
+    }
+  }
+  if (tid == 0) *s_back = 0;
+  __syncthreads();
+  if (tid == 0) {
+    const S rsj = st->rs[j];
+    const double eps = st->eps, tolr = st->tolr;
+    const int kdim = st->kdim, maxits = st->maxits, iter = st->iter + 1;
+    h[j + 1] = S(t);
+    st->sc[j + 1] = 1.0 / t;
+    st->iter = iter;
+    st->i = j + 1;
+    for (int k = 1; k <= j; k++) {
+      const S hii = h[k - 1], hk = h[k];
+      h[k - 1] = conj(rc[k - 1]) * hii + rs_[k - 1] * hk;
+      h[k] = -rs_[k - 1] * hii + rc[k - 1] * hk;
+    }
+    const S hii = h[j], hii1 = h[j + 1];
+    const double gam = sqrt(cabs(hii) * cabs(hii) + cabs(hii1) * cabs(hii1));
+    if (fabs(gam) < eps) {
+      st->hist[j] = 0.0;
+      st->breakdown = 1;
+      st->i = 0;
+      st->cycle_done = 1;
+      st->done = 1;
+    } else {
+      const S c = hii / gam, s = hii1 / gam;
+      st->c[j] = c;
+      st->s[j] = s;
+      const S next = -s * rsj;
+      st->rs[j + 1] = next;
+      st->rs[j] = conj(c) * rsj;
+      h[j] = conj(c) * hii + s * hii1;
+      const double normr = cabs(next);
+      st->normr = normr;
+      st->hist[j] = normr;
+      const bool conv = normr <= tolr;
+      if (conv) st->converged = 1;
+      if (conv || j + 1 >= kdim || iter >= maxits) {
+        st->cycle_done = 1;
+        if (conv || iter >= maxits) st->done = 1;
+        *s_back = j + 1;
+      }
+    }
+  }
+  __syncthreads();
+  for (int c = tid; c <= j + 1; c += blockDim.x) st->H[(size_t)j * ldh + c] = h[c];
+  const int n = *s_back;
+  if (n == 0) return;
+  __syncthreads();  // rs and the last column of H are written
+  if (tid < 32) {
+    constexpr int Q = (KMAX + 31) / 32;
+    S r[Q], col[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const int i = tid + 32 * q;
+      r[q] = i < n ? st->rs[i] : S(0.0);
+      col[q] = i < n ? st->H[(size_t)(n - 1) * ldh + i] : S(0.0);
+    }
+    for (int k = n - 1; k >= 0; k--) {
+      S nxt[Q];
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const int i = tid + 32 * q;
+        nxt[q] = k > 0 && i < k ? st->H[(size_t)(k - 1) * ldh + i] : S(0.0);
+      }
+      S rk = S(0.0), d = S(0.0);
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+        if (k / 32 == q) {
+          rk = r[q];
+          d = col[q];
+        }
+      const S y = bcast(rk, k & 31) / bcast(d, k & 31);
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const int i = tid + 32 * q;
+        if (i < k) r[q] -= col[q] * y;
+        if (i == k) r[q] = y;
+        col[q] = nxt[q];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+      if (tid + 32 * q < n) st->rs[tid + 32 * q] = r[q];
+  }
+}
+
 template <typename TV, typename TM, typename TW>
-__device__ inline void ts_epilogue(const TsArgs<TV, TM, TW>& a, const TsAcc<TW>* sums, int ncols) {
+__device__ inline void ts_epilogue(const TsArgs<TV, TM, TW>& a, const TsAcc<TW>* sums) {
   using A = TsAcc<TW>;
   FgmresDevT<A>* st = a.st;
   switch (a.epi) {
-    case EPI_STORE:
-      for (int c = 0; c < ncols; c++) a.dst[c] = sums[c] * (a.vsc ? a.vsc[c] : 1.0);
-      break;
-    case EPI_CGS_FIRST:
-      for (int c = 0; c < ncols; c++) {
-        A h = sums[c] * (a.vsc ? a.vsc[c] : 1.0);
-        st->hcol[c] = h;
-        st->coefA[c] = h;
-      }
-      break;
-    case EPI_CGS_SECOND:
-      for (int c = 0; c < ncols; c++) {
-        A h = sums[c] * (a.vsc ? a.vsc[c] : 1.0);
-        st->hcol[c] += h;
-        st->coefB[c] = h;
-      }
-      break;
-    case EPI_GIVENS:
-      fgmres_givens(st, a.j, sqrt(re(sums[0])));
-      break;
     case EPI_NORMB:
       st->normb = sqrt(re(sums[0]));
       if (st->normb < st->eps) {
@@ -1070,7 +1186,7 @@ __device__ inline void ts_epilogue(const TsArgs<TV, TM, TW>& a, const TsAcc<TW>*
 }
 
 template <typename TV, typename TM, typename TW, int MODE>
-__global__ void __launch_bounds__(kTsThreads) ts_kernel(TsArgs<TV, TM, TW> a) {
+__device__ __forceinline__ void ts_body(const TsArgs<TV, TM, TW>& a) {
   using A = TsAcc<TW>;
   if (a.skip.on()) return;
   __shared__ A scoef[KMAX + 1];
@@ -1097,21 +1213,21 @@ __global__ void __launch_bounds__(kTsThreads) ts_kernel(TsArgs<TV, TM, TW> a) {
     const int row = r0 + tid;
     A wv = A(0.0);
     if (row < a.n) {
-      wv = a.in ? to<A>(a.in[row]) * in_s : A(0.0);
+      wv = a.in ? mul_rn(to<A>(a.in[row]), in_s) : A(0.0);
       if (update) {
         A acc = A(0.0);
         const TM* m = a.M + row;
-        for (int c = 0; c < ncols; c++) acc += to<A>(m[(long long)c * a.ldm]) * scoef[c];
+        for (int c = 0; c < ncols; c++) mac(acc, to<A>(m[(long long)c * a.ldm]), scoef[c]);
         wv += acc;
       }
       if (MODE != TS_DOT && a.out) a.out[row] = to<TW>(wv);
     }
     if (MODE == TS_UPDATE_NORM || MODE == TS_NORM_COPY) {
-      double sq = (row < a.n) ? abs2(wv) : 0.0;
+      double sq = (row < a.n) ? abs2_rn(wv) : 0.0;
       if (MODE == TS_UPDATE_NORM) {
         // the norm of the stored (rounded) vector, as Norm2 of the reference
         TW stored = to<TW>(wv);
-        sq = (row < a.n) ? abs2(to<A>(stored)) : 0.0;
+        sq = (row < a.n) ? abs2_rn(to<A>(stored)) : 0.0;
       }
       sq = warp_reduce(sq);
       if (lane == 0) swarp[warp] += sq;  // one writer per slot: deterministic
@@ -1123,8 +1239,8 @@ __global__ void __launch_bounds__(kTsThreads) ts_kernel(TsArgs<TV, TM, TW> a) {
         const TV* v = a.V + (long long)c * a.ldv + r0;
         A acc = A(0.0);
         for (int k = lane; k < nrows_tile; k += 32) {
-          A w = (MODE == TS_DOT) ? (a.in ? to<A>(a.in[r0 + k]) * in_s : A(0.0)) : to<A>(a.out[r0 + k]);
-          acc += conj(to<A>(v[k])) * w;
+          A w = (MODE == TS_DOT) ? (a.in ? mul_rn(to<A>(a.in[r0 + k]), in_s) : A(0.0)) : to<A>(a.out[r0 + k]);
+          mac(acc, conj(to<A>(v[k])), w);
         }
         acc = warp_reduce(acc);
         if (lane == 0) sacc[c] += acc;
@@ -1158,21 +1274,98 @@ __global__ void __launch_bounds__(kTsThreads) ts_kernel(TsArgs<TV, TM, TW> a) {
     if (lane == 0) sacc[c] = acc;
   }
   __syncthreads();
-  if (tid == 0) {
-    ts_epilogue(a, sacc, nred);
-    *a.counter = 0u;
-    __threadfence();
+  switch (a.epi) {
+    case EPI_STORE:
+      for (int c = tid; c < nred; c += kTsThreads) a.dst[c] = sacc[c] * (a.vsc ? a.vsc[c] : 1.0);
+      break;
+    case EPI_CGS_FIRST:
+      for (int c = tid; c < nred; c += kTsThreads) {
+        const A h = sacc[c] * (a.vsc ? a.vsc[c] : 1.0);
+        a.st->hcol[c] = h;
+        a.st->coefA[c] = h;
+      }
+      break;
+    case EPI_CGS_SECOND:
+      for (int c = tid; c < nred; c += kTsThreads) {
+        const A h = sacc[c] * (a.vsc ? a.vsc[c] : 1.0);
+        a.st->hcol[c] += h;
+        a.st->coefB[c] = h;
+      }
+      break;
+    case EPI_GIVENS:
+      // only the kernel that ends a Krylov step carries this code
+      if constexpr (MODE == TS_UPDATE_NORM) {
+        __shared__ A sgiv[3 * (KMAX + 1)];
+        __shared__ int s_back;
+        fgmres_givens_block(a.st, a.j, sqrt(re(sacc[0])), sgiv, &s_back);
+      }
+      break;
+    default:
+      if (tid == 0) ts_epilogue(a, sacc);
+      break;
   }
+  if (tid == 0) *a.counter = 0u;
+  __threadfence();
+}
+
+template <typename TV, typename TM, typename TW, int MODE>
+__global__ void __launch_bounds__(kTsThreads) ts_kernel(const __grid_constant__ TsArgs<TV, TM, TW> a) {
+  ts_body<TV, TM, TW, MODE>(a);
+}
+
+// The kernels of a multi-lane slot: one launch for all lanes, lane
+// blockIdx.y with the arguments, grid and sums of its own single launch.
+// Most of these kernels work on a few thousand rows and are bound by their
+// launch: 16 right-hand sides of a complex 24^3 problem as one block took
+// 198 ms with a launch per lane and take 58 ms (B200); 24 at 48^3, four to a
+// slot, 131 and 86 ms.
+template <typename TV, typename TM, typename TW>
+struct TsLanes {
+  TsArgs<TV, TM, TW> a[kMaxLanes];
+};
+template <typename TV, typename TM, typename TW, int MODE>
+__global__ void __launch_bounds__(kTsThreads) ts_lanes_kernel(const __grid_constant__ TsLanes<TV, TM, TW> p) {
+  ts_body<TV, TM, TW, MODE>(p.a[blockIdx.y]);
+}
+
+template <typename TX, typename TY>
+struct SpmvLanes {
+  const TX *x1[kMaxLanes], *x2[kMaxLanes];
+  const TY* b[kMaxLanes];
+  TY* y[kMaxLanes];
+  int* err[kMaxLanes];
+  Skip skip[kMaxLanes];
+};
+template <typename TA, typename TX, typename TY, typename TC, int S>
+__global__ void __launch_bounds__(256) spmv_lanes_kernel(
+    int nrows, const int* __restrict__ rp1, const int* __restrict__ cj1, const TA* __restrict__ va1, int xcols1,
+    TC alpha, const int* __restrict__ rp2, const int* __restrict__ cj2, const TA* __restrict__ va2, int xcols2,
+    TC alpha2, TC beta, const __grid_constant__ SpmvLanes<TX, TY> p) {
+  const int r = blockIdx.y;
+  if (p.skip[r].on()) return;
+  spmv_rows<TA, TX, TY, TC, S, true>(nrows, rp1, cj1, va1, p.x1[r], xcols1, alpha, rp2, cj2, va2, p.x2[r], xcols2,
+                                     alpha2, p.b[r], beta, p.y[r], nullptr, p.err[r]);
 }
 
 template <typename S>
-__global__ void fgmres_cycle_reset_kernel(FgmresDevT<S>* st, Skip skip) {
-  if (skip.on()) return;
+struct StateLanes {
+  FgmresDevT<S>* st[kMaxLanes];
+};
+template <typename S>
+__device__ __forceinline__ void fgmres_cycle_reset(FgmresDevT<S>* st) {
   st->i = 0;
   if (st->done) return;
   st->cycle_done = 0;
   st->rs[0] = S(st->normr);
   st->sc[0] = 1.0 / st->normr;
+}
+template <typename S>
+__global__ void fgmres_cycle_reset_kernel(FgmresDevT<S>* st, Skip skip) {
+  if (!skip.on()) fgmres_cycle_reset(st);
+}
+template <typename S>
+__global__ void fgmres_cycle_reset_lanes_kernel(const __grid_constant__ StateLanes<S> p) {
+  fgmres_cycle_reset(p.st[threadIdx.x]);
 }
 
 // --------------------------------------------------- permutation + convert
@@ -1182,10 +1375,15 @@ __global__ void fgmres_cycle_reset_kernel(FgmresDevT<S>* st, Skip skip) {
 // dependent loads of several entries are in flight together.
 constexpr int kPermUnroll = 4;
 template <typename TI, typename TO>
-__global__ void __launch_bounds__(256) gather_kernel(int n, const int* __restrict__ perm, const TI* __restrict__ in,
-                                                     const double* __restrict__ scale, TO* __restrict__ out,
-                                                     Skip skip) {
-  if (skip.on()) return;
+struct PermLanes {
+  const TI* in[kMaxLanes];
+  const double* scale[kMaxLanes];
+  TO* out[kMaxLanes];
+  Skip skip[kMaxLanes];
+};
+template <typename TI, typename TO>
+__device__ __forceinline__ void gather_rows(int n, const int* __restrict__ perm, const TI* __restrict__ in,
+                                            const double* __restrict__ scale, TO* __restrict__ out) {
   const double s = scale ? *scale : 1.0;
   const int stride = gridDim.x * blockDim.x * kPermUnroll;
   for (int base = blockIdx.x * blockDim.x * kPermUnroll + threadIdx.x; base < n; base += stride) {
@@ -1206,6 +1404,19 @@ __global__ void __launch_bounds__(256) gather_kernel(int n, const int* __restric
   }
 }
 
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256) gather_kernel(int n, const int* __restrict__ perm, const TI* __restrict__ in,
+                                                     const double* __restrict__ scale, TO* __restrict__ out,
+                                                     Skip skip) {
+  if (!skip.on()) gather_rows<TI, TO>(n, perm, in, scale, out);
+}
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256) gather_lanes_kernel(int n, const int* __restrict__ perm,
+                                                           const __grid_constant__ PermLanes<TI, TO> p) {
+  const int r = blockIdx.y;
+  if (!p.skip[r].on()) gather_rows<TI, TO>(n, perm, p.in[r], p.scale[r], p.out[r]);
+}
+
 // y += x  (the solution update of the multiplicative level solve)
 template <typename T>
 __global__ void __launch_bounds__(256) axpy_kernel(int n, const T* __restrict__ x, T* __restrict__ y, Skip skip) {
@@ -1215,9 +1426,8 @@ __global__ void __launch_bounds__(256) axpy_kernel(int n, const T* __restrict__ 
 
 // out[perm[i]] = in[i]  (IntVectorClass::ScatterRperm, int_vector.cpp:629)
 template <typename TI, typename TO>
-__global__ void __launch_bounds__(256) scatter_kernel(int n, const int* __restrict__ perm, const TI* __restrict__ in,
-                                                      TO* __restrict__ out, Skip skip) {
-  if (skip.on()) return;
+__device__ __forceinline__ void scatter_rows(int n, const int* __restrict__ perm, const TI* __restrict__ in,
+                                             TO* __restrict__ out) {
   const int stride = gridDim.x * blockDim.x * kPermUnroll;
   for (int base = blockIdx.x * blockDim.x * kPermUnroll + threadIdx.x; base < n; base += stride) {
     int p[kPermUnroll];
@@ -1232,6 +1442,18 @@ __global__ void __launch_bounds__(256) scatter_kernel(int n, const int* __restri
     for (int u = 0; u < kPermUnroll; u++)
       if (p[u] >= 0) out[p[u]] = to<TO>(v[u]);
   }
+}
+
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256) scatter_kernel(int n, const int* __restrict__ perm, const TI* __restrict__ in,
+                                                      TO* __restrict__ out, Skip skip) {
+  if (!skip.on()) scatter_rows<TI, TO>(n, perm, in, out);
+}
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256) scatter_lanes_kernel(int n, const int* __restrict__ perm,
+                                                            const __grid_constant__ PermLanes<TI, TO> p) {
+  const int r = blockIdx.y;
+  if (!p.skip[r].on()) scatter_rows<TI, TO>(n, perm, p.in[r], p.out[r]);
 }
 
 template <typename T>
