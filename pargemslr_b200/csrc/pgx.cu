@@ -31,6 +31,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <exception>
+#include <complex>
 #include <mutex>
 #include <new>
 #include <string>
@@ -179,19 +180,24 @@ struct HostLevel {
 // rows ordered by level, then by index (IluClass::BuildLevels,
 // ParGeMSLR SRC/preconditioners/ilu.cpp:832-1062).  Lower factors are swept
 // from the first row, upper factors from the last.
+static int check_triangular(bool upper, int n, const int* rp, const int* cj) {
+  for (int i = 0; i < n; i++)
+    for (int k = rp[i]; k < rp[i + 1]; k++)
+      if (upper ? cj[k] <= i : cj[k] >= i)
+        return fail(PGX_ERROR_INVALID_PARAM, "%s factor is not strictly %s triangular (row %d, col %d)",
+                    upper ? "U" : "L", upper ? "upper" : "lower", i, cj[k]);
+  return PGX_SUCCESS;
+}
 static int build_levels(bool upper, int n, const int* rp, const int* cj, std::vector<int>& level_ptr,
                         std::vector<int>& order, std::vector<int>* lev_out = nullptr) {
+  PGX_TRY(check_triangular(upper, n, rp, cj));
   std::vector<int> lev(n, -1);
   int max_level = 0;
   for (int t = 0; t < n; t++) {
     int i = upper ? n - 1 - t : t;
     int l = -1;
     for (int k = rp[i]; k < rp[i + 1]; k++) {
-      int j = cj[k];
-      if (upper ? (j <= i) : (j >= i))
-        return fail(PGX_ERROR_INVALID_PARAM, "%s factor is not strictly %s triangular (row %d, col %d)",
-                    upper ? "U" : "L", upper ? "upper" : "lower", i, j);
-      l = std::max(l, lev[j]);
+      l = std::max(l, lev[cj[k]]);
     }
     lev[i] = l + 1;
     max_level = std::max(max_level, lev[i]);
@@ -649,10 +655,94 @@ static bool want_segments(const HostCsr& h, int nnz_cap) {
   return maxlen <= nnz_cap - 4 && avg * 32.0 <= (double)nnz_cap;
 }
 
+// The product of both inverse factors, M = U^-1 D L^-1 (rows of `vw` doubles a
+// value), when the factors are shallow: at most kDirectLevels dependency
+// levels each, and M no longer than twice the factors.  Lower levels of a
+// hierarchy hold separators that hardly couple (3,000 rows, under 100
+// entries, one to four levels at 64^3): their B-solve is then one product
+// instead of two passes: ncu on a B200, 64^3 mixed, 6 us for the product, 19
+// us for each pass, 25 B-solves of this kind a preconditioner call.  Entries
+// are formed in FP64 and rounded once.
+constexpr int kDirectLevels = 8;
+template <typename S>
+static bool shallow_inverse(const HostCsr& L, const HostCsr& U, const std::vector<double>& dinv, HostCsr& M) {
+  const int n = L.rows;
+  constexpr int vw = sizeof(S) / sizeof(double);
+  if (n == 0 || U.rows != n || (int)dinv.size() < n * vw) return false;
+  for (const HostCsr* T : {&L, &U}) {
+    std::vector<int> lev(n, 0);
+    for (int t = 0; t < n; t++) {
+      const int i = T == &U ? n - 1 - t : t;
+      for (int k = T->rp[i]; k < T->rp[i + 1]; k++) lev[i] = std::max(lev[i], lev[T->cj[k]] + 1);
+      if (lev[i] >= kDirectLevels) return false;
+    }
+  }
+  const size_t limit = 2 * ((size_t)n + (size_t)L.nnz() + (size_t)U.nnz());
+  const S *lv = (const S*)L.va.data(), *uv = (const S*)U.va.data(), *dv = (const S*)dinv.data();
+  // rows of an inverse, formed in solving order: row_i = d_i (e_i - sum_j T_ij row_j)
+  std::vector<S> acc(n, S(0));
+  std::vector<char> in(n, 0);
+  std::vector<int> touched;
+  using Rows = std::vector<std::vector<std::pair<int, S>>>;
+  auto add = [&](int j, const S& v) {
+    if (!in[j]) {
+      in[j] = 1;
+      touched.push_back(j);
+      acc[j] = v;
+    } else {
+      acc[j] += v;
+    }
+  };
+  auto take = [&](std::vector<std::pair<int, S>>& row, size_t& count) {
+    std::sort(touched.begin(), touched.end());
+    for (int j : touched) {
+      row.push_back({j, acc[j]});
+      in[j] = 0;
+    }
+    count += touched.size();
+    touched.clear();
+    return count <= limit;
+  };
+  Rows li(n), ui(n);
+  size_t count = 0;
+  for (int i = 0; i < n; i++) {
+    for (int k = L.rp[i]; k < L.rp[i + 1]; k++)
+      for (const auto& e : li[L.cj[k]]) add(e.first, -(lv[k] * e.second));
+    add(i, S(1.0));
+    if (!take(li[i], count)) return false;
+  }
+  count = 0;
+  for (int i = n - 1; i >= 0; i--) {
+    for (int k = U.rp[i]; k < U.rp[i + 1]; k++)
+      for (const auto& e : ui[U.cj[k]]) add(e.first, -(dv[i] * uv[k] * e.second));
+    add(i, dv[i]);
+    if (!take(ui[i], count)) return false;
+  }
+  M = HostCsr();
+  M.rows = M.cols = n;
+  M.rp.assign(1, 0);
+  count = 0;
+  std::vector<std::pair<int, S>> row;
+  for (int i = 0; i < n; i++) {
+    for (const auto& u : ui[i])
+      for (const auto& e : li[u.first]) add(e.first, u.second * e.second);
+    row.clear();
+    if (!take(row, count)) return false;
+    for (const auto& e : row) {
+      M.cj.push_back(e.first);
+      const double* v = (const double*)&e.second;
+      M.va.insert(M.va.end(), v, v + vw);
+    }
+    M.rp.push_back((int)M.cj.size());
+  }
+  return true;
+}
+
 template <typename P>
 struct DLevel {
   int start = 0, nl = 0, m = 0, rank = 0;
   DTri<P> L, U;
+  DCsr<P> inv;  // shallow factors: the product of their inverses, in place of L and U
   P* dinv = nullptr;
   P* y = nullptr;  // lower-pass result, holds the sentinel between solves
   P* yslot = nullptr;  // lower-pass result in the upper pass's slot order (per-subdomain kernels)
@@ -986,8 +1076,16 @@ struct Engine : EngineBase {
       d.start = lev_ptr[l];
       d.nl = lev_ptr[l + 1] - lev_ptr[l];
       d.m = n - lev_ptr[l + 1];
+      PGX_TRY(check_triangular(false, h.L.rows, h.L.rp.data(), h.L.cj.data()));
+      PGX_TRY(check_triangular(true, h.U.rows, h.U.rp.data(), h.U.cj.data()));
+      HostCsr inv;
+      const bool direct = im.vw == 2 ? shallow_inverse<std::complex<double>>(h.L, h.U, h.dinv, inv)
+                                     : shallow_inverse<double>(h.L, h.U, h.dinv, inv);
       int rcL = PGX_ERROR_INVALID_PARAM, rcU = PGX_ERROR_INVALID_PARAM;
-      if (h.L.rows > 0) {
+      if (direct) {
+        PGX_TRY(upload_csr(ar, inv, d.inv, stream));
+        rcL = rcU = PGX_SUCCESS;
+      } else if (h.L.rows > 0) {
         std::vector<int> uslot_of_row;
         rcU = upload_tri_flow<P, 1>(ar, h.U, true, h.dom_ptr, d.U, stream, &h.dinv, &uslot_of_row, nullptr);
         if (rcU == PGX_SUCCESS)
@@ -1092,6 +1190,7 @@ struct Engine : EngineBase {
     for (int l = 0; l < nlev; l++) {
       need(lv[l].E);
       need(lv[l].F);
+      need(lv[l].inv);
     }
     need(C0);
     if (mthreads > 0) {
@@ -1458,6 +1557,10 @@ struct Engine : EngineBase {
   // B-solve of level l: x = U^-1 L^-1 rhs  (GemslrClass::SolveB)
   void solve_b(int l, const P* rhs, const double* rhs_scale, P* x, Skip sk) {
     DLevel<P>& d = lv[l];
+    if (d.inv.rows > 0) {
+      spmv<P, P, P, P>(d.inv, rhs, (P)1, nullptr, nullptr, (P)0, (const P*)nullptr, (P)0, x, rhs_scale, sk);
+      return;
+    }
     trsv(d.L, false, nullptr, rhs, rhs_scale, d.y, x, sk, d.yslot);
     trsv(d.U, true, d.dinv, nullptr, nullptr, d.y, x, sk, d.yslot);
   }
@@ -1685,14 +1788,17 @@ struct Engine : EngineBase {
     if (which <= 1) {
       DLevel<P>& d = lv[level];
       const DTri<P>& T = which == 0 ? d.L : d.U;
-      const double nnz = (double)(which == 0 ? d.L.nnz_total : d.U.nnz_total);
+      const double nnz = (double)(d.inv.rows > 0 ? d.inv.nnz : which == 0 ? d.L.nnz_total : d.U.nnz_total);
       *bytes = nnz * (vb + 4.0) + 4.0 * (d.nl + 1) + 4.0 * d.nl + 2.0 * vb * d.nl + (which == 1 ? vb * d.nl : 0.0);
-      *launches = T.n > 0 ? 1 : 0;
+      *launches = T.n > 0 || (which == 0 && d.inv.rows > 0) ? 1 : 0;
       // lower and upper passes alternate so the sentinel protocol stays valid;
       // the events bracket only the pass being measured
       for (int r = 0; r < reps; r++) {
         if (which == 0) PGX_CUDA(cudaEventRecord(ev0, stream));
-        trsv(d.L, false, nullptr, rt, nullptr, d.y, xt, sk, d.yslot);
+        if (d.inv.rows > 0)
+          solve_b(level, rt, nullptr, xt, sk);  // one product for both passes, counted as the lower one
+        else
+          trsv(d.L, false, nullptr, rt, nullptr, d.y, xt, sk, d.yslot);
         if (which == 0) PGX_CUDA(cudaEventRecord(ev1, stream));
         if (which == 1) PGX_CUDA(cudaEventRecord(ev0, stream));
         trsv(d.U, true, d.dinv, nullptr, nullptr, d.y, xt, sk, d.yslot);
@@ -1997,8 +2103,12 @@ struct Engine : EngineBase {
       const DLevel<P>& d = lv[l];
       snprintf(buf, sizeof(buf), "level %d: rows %d, trailing %d, rank %d\n", l, d.nl, d.m, d.rank);
       o += buf;
-      o += describe_tri("L", d.L);
-      o += describe_tri("U", d.U);
+      if (d.inv.rows > 0) {
+        o += describe_csr("L, U: product of the inverses", d.inv);
+      } else {
+        o += describe_tri("L", d.L);
+        o += describe_tri("U", d.U);
+      }
       o += describe_csr("E", d.E);
       o += describe_csr("F", d.F);
     }
@@ -2411,6 +2521,12 @@ struct BatchEngine : EngineBase {
 
   void solve_b_b(int l, const std::array<const P*, R>& rhs, const std::array<P*, R>& x,
                  const std::array<Skip, R>& sk) {
+    const DLevel<P>& d = lane[0]->lv[l];
+    if (d.inv.rows > 0) {
+      spmv_b<P, P, P, P>(d.inv, rhs, (P)1, nullptr, (const std::array<const P*, R>*)nullptr, (P)0,
+                         (const std::array<const P*, R>*)nullptr, (P)0, x, sk);
+      return;
+    }
     std::array<P*, R> y;
     std::array<const P*, R> none;
     for (int r = 0; r < R; r++) {
@@ -2875,7 +2991,10 @@ struct BatchEngine : EngineBase {
     float total = 0.f;
     for (int rep = 0; rep < reps; rep++) {
       if (which == 0) PGX_CUDA(cudaEventRecord(e0, stream));
-      trsv_b(level, false, rt, y, xt, sk);
+      if (lane[0]->lv[level].inv.rows > 0)
+        solve_b_b(level, rt, xt, sk);
+      else
+        trsv_b(level, false, rt, y, xt, sk);
       if (which == 0) PGX_CUDA(cudaEventRecord(e1, stream));
       if (which == 1) PGX_CUDA(cudaEventRecord(e0, stream));
       trsv_b(level, true, none, y, xt, sk);

@@ -45,7 +45,8 @@ CASES = {
     "one row": ([0, 1], 0, 1, 0),
     "a task and a row": ([0, 33], 3, 20, 0),
     "diagonal": ([0, 1300], 0, 1, 0),
-    "chain": ([0, 400], 1, 1, 0),
+    "chains": ([0, 400], 1, 1, 0),
+    "a row a level": ([0, 300], 3, 2, 0),
     "two narrow subdomains and an empty one": ([0, 517, 517, 900], 6, 40, 0),
     "long rows": ([0, 2500], 6, 150, 90),
     "ring wraps": ([0, 20000], 4, 30, 0),
@@ -69,7 +70,10 @@ def test_pass_pair(name, cplx, precision):
     b = rng.standard_normal(n) + (1j * rng.standard_normal(n) if cplx else 0.0)
     h = GemslrHandle(st, precision=precision)
     try:
-        assert "dataflow" in h.describe()
+        if name in ("one row", "diagonal"):
+            assert "product of the inverses" in h.describe()
+        elif name not in ("a task and a row", "chains"):  # those are about as deep as the limit
+            assert "dataflow" in h.describe()
         z = h.apply(b)
     finally:
         h.close()
@@ -77,3 +81,54 @@ def test_pass_pair(name, cplx, precision):
     # |x| stays of order |b| (row sums of the factors are below 1): rounding of 90 products a row at most
     tol = 1e-13 if precision == "fp64" else 2e-5
     assert np.linalg.norm(z - ref) <= tol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("levels", [2, 7, 8, 9])
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+def test_shallow_factors(levels, cplx):
+    """Factors on both sides of the depth at which one product takes the place of the two passes."""
+    from pargemslr_b200.handle import GemslrHandle
+    n, seps = 999, 999 // levels
+    rng = np.random.default_rng(levels)
+    rp = np.zeros(n + 1, np.int32)
+    coupled = np.arange(n) % seps == 3  # a few chains of `levels` rows
+    rows = np.flatnonzero(coupled)[1:levels]
+    rp[rows + 1] = 1
+    rp = np.cumsum(rp).astype(np.int32)
+    cj = (rows - seps).astype(np.int32)
+    va = rng.uniform(-1, 1, len(rows)) + (1j * rng.uniform(-1, 1, len(rows)) if cplx else 0.0)
+    L = (rp, cj, va, n, n)
+    up = np.zeros(n + 1, np.int32)
+    up[cj + 1] = 1
+    U = (np.cumsum(up).astype(np.int32), rows.astype(np.int32), va[::-1].copy(), n, n)
+    dinv = 1.0 + rng.random(n) + (0.3j if cplx else 0.0)
+    eye = (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n, dinv.dtype), n, n)
+    lv = LevelStructures(ncomp=1, dom_ptr=np.array([0, n], np.int32), L=L, U=U, dinv=dinv, B=eye)
+    st = GemslrStructures(n=n, A=eye, pperm=np.arange(n, dtype=np.int32), qperm=None,
+                          lev_ptr=np.array([0, n], np.int32), levels=[lv], inner_enable=0)
+    b = rng.standard_normal(n) + (1j * rng.standard_normal(n) if cplx else 0.0)
+    h = GemslrHandle(st, precision="fp64")
+    try:
+        assert ("product of the inverses" in h.describe()) == (levels <= 8)
+        z = h.apply(b)
+    finally:
+        h.close()
+    ref = _substitute(L, U, dinv, b)
+    assert np.linalg.norm(z - ref) <= 1e-14 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("bad", ["L", "U"])
+def test_factor_that_is_not_triangular_is_refused(bad):
+    from pargemslr_b200 import _abi
+    from pargemslr_b200.handle import GemslrHandle
+    n = 40
+    eye = (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n), n, n)
+    lv = LevelStructures(ncomp=1, dom_ptr=np.array([0, n], np.int32), L=empty_csr(n, n), U=empty_csr(n, n),
+                         dinv=np.ones(n), B=eye)
+    rp = np.zeros(n + 1, np.int32)
+    rp[8:] = 1  # one entry, in row 7
+    setattr(lv, bad, (rp, np.array([9 if bad == "L" else 5], np.int32), np.ones(1), n, n))
+    st = GemslrStructures(n=n, A=eye, pperm=np.arange(n, dtype=np.int32), qperm=None,
+                          lev_ptr=np.array([0, n], np.int32), levels=[lv], inner_enable=0)
+    with pytest.raises(_abi.PgxError, match="triangular"):
+        GemslrHandle(st, precision="fp64").close()
