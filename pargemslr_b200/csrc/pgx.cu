@@ -603,9 +603,10 @@ static int upload_tri_flow(Arena& ar, const HostCsr& h, bool upper, const std::v
   const bool fits = flow_pack<T, C>(n, h.rp.data(), h.cj.data(), val, upper, cuts, &diag, upper_slot_of_row, pk);
   // Operands that left the ring are read back from global memory.  When they
   // are more than a hundredth of the entries, a ring twice as long with fewer
-  // warps is the better trade (FP64, four lanes: 128^3, 30% of the entries
-  // far, 19.7 ms against 11.4 ms with the longer ring; 64^3, 0.1% far, 1.00
-  // ms against 1.14 ms).
+  // warps is the better trade.  128^3, lower pass on a B200: four lanes mixed,
+  // 2.6% far, 6.7 ms, with the longer ring 4.6 ms; one lane FP64, 2.5% far, 5.2
+  // and 4.2 ms; one lane mixed, 0.1% far, 2.0 and 2.2 ms.  64^3, four lanes
+  // mixed, 0.04% far: 0.47 and 0.63 ms.
   d.flow_long = false;
   if constexpr (C::has_long) {
     if (!fits || pk.nfar * 100 > h.nnz()) {

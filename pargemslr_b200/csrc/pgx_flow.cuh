@@ -22,9 +22,10 @@
 //     a CTA barrier a level took 600-900.)
 //   - one more warp streams the factor into shared memory by bulk copies.
 // On a B200, level 0 of the 7-point Laplacian at 64^3 (ILUT 1e-3), lower /
-// upper pass: 0.30 / 0.30 ms mixed and 0.46 / 0.43 ms FP64, one lane (one
-// barrier a level: 1.30 / 1.19 and 1.64 / 1.52 ms); 0.46 / 0.43 ms for four
-// lanes mixed.  At 128^3, mixed: 2.0 / 1.9 ms one lane (6.04 / 5.76).
+// upper pass: 0.29 / 0.28 ms mixed and 0.46 / 0.43 ms FP64, one lane (one
+// barrier a level: 1.30 / 1.19 and 1.64 / 1.52 ms); 0.47 / 0.45 ms for four
+// lanes mixed.  At 128^3, mixed: 2.0 / 1.8 ms one lane (6.04 / 5.76), 4.6 /
+// 4.0 ms four lanes.
 #pragma once
 
 #include "pgx_device.cuh"
@@ -33,18 +34,6 @@
 namespace pgx {
 
 constexpr int kFlowPolls = 1 << 23;      // bound of a wait, in polls
-
-template <typename T>
-__device__ __forceinline__ void flow_mac(T& acc, T v, T w) {
-  if constexpr (Sc<T>::complex) {
-    acc.x = fma(v.x, w.x, acc.x);
-    acc.y = fma(v.x, w.y, acc.y);
-    acc.x = fma(-v.y, w.y, acc.x);
-    acc.y = fma(v.y, w.x, acc.y);
-  } else {
-    acc = fma(v, w, acc);
-  }
-}
 
 struct FlowArgs {
   int n;                    // rows; also the length of the slot vector
@@ -289,28 +278,58 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
 #pragma unroll
       for (int r = 0; r < R; r++) b[r] = UPPER ? ldcg(&yslot.p[r][h3.w + l]) : ldcg(&rhs.p[r][id]);
     }
-    T acc0[R], acc1[R];
+    T acc[kFlowSets<T>][4][R], last[2][R];  // the last quad's sums: entries 0 and 1, entries 2 and 3
 #pragma unroll
-    for (int r = 0; r < R; r++) acc0[r] = acc1[r] = T(0);
+    for (int r = 0; r < R; r++) last[0][r] = last[1][r] = T(0);
+#pragma unroll
+    for (int e = 0; e < kFlowSets<T>; e++)
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[e][u][r] = T(0);
     // far operands: solved so long ago that they left the ring.  Their tasks
     // are 3 W back: this warp's last wait covers the release after their stores.
-    if (h3.x > 0) {
-      for (int q = 0; q < h3.x; q++) {
-        const int4 fc = *(const int4*)(base + h3.y + (size_t)(q * stride + l) * 16);
-        const T* fv = (const T*)(base + h3.y + (size_t)h3.x * stride * 16 + (size_t)(q * stride + l) * 4 * sizeof(T));
-        const int cc[4] = {fc.x, fc.y, fc.z, fc.w};
-        T w[4][R];
+    constexpr int FQ = R == 1 ? 2 : 1;  // far quads whose loads are in flight together
+    for (int q0 = 0; q0 < h3.x; q0 += FQ) {
+      int cc[FQ][4];
+      T fv[FQ][4], w[FQ][4][R];
+#pragma unroll
+      for (int e = 0; e < FQ; e++) {
+        const bool have = q0 + e < h3.x;
+        const size_t at = (size_t)((have ? q0 + e : q0) * stride + l);
+        const int4 fc = *(const int4*)(base + h3.y + at * 16);
+        const T* vp = (const T*)(base + h3.y + (size_t)h3.x * stride * 16 + at * 4 * sizeof(T));
+        cc[e][0] = have ? fc.x : -1;
+        cc[e][1] = have ? fc.y : -1;
+        cc[e][2] = have ? fc.z : -1;
+        cc[e][3] = have ? fc.w : -1;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          const bool in = (unsigned)cc[u] < (unsigned)a.n;
+          const int j = cc[e][u] & kFlowIndex;
+          const bool in = cc[e][u] >= 0 && j < a.n;
+          fv[e][u] = in ? vp[u] : T(0);
 #pragma unroll
-          for (int r = 0; r < R; r++) w[u][r] = in ? ldcg(UPPER ? &x.p[r][cc[u]] : &yslot.p[r][cc[u]]) : T(0);
+          for (int r = 0; r < R; r++) w[e][u][r] = in ? ldcg(UPPER ? &x.p[r][j] : &yslot.p[r][j]) : T(0);
         }
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-          for (int r = 0; r < R; r++) flow_mac(u & 1 ? acc1[r] : acc0[r], fv[u], w[u][r]);
       }
+#pragma unroll
+      for (int e = 0; e < FQ; e++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const bool newest = (cc[e][u] & kFlowLast) != 0;
+          const bool other = kFlowSets<T> == 2 && (cc[e][u] & kFlowOther);
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            T t = newest ? last[u / 2][r] : other ? acc[kFlowSets<T> - 1][u][r] : acc[0][u][r];
+            mac(t, fv[e][u], w[e][u][r]);
+            if (newest)
+              last[u / 2][r] = t;
+            else if (other)
+              acc[kFlowSets<T> - 1][u][r] = t;
+            else
+              acc[0][u][r] = t;
+          }
+        }
     }
     flow_wait<C::W>(s_prog, h1.y, lane, err, &s_abort);
     // the slots of the rows half a ring ahead: their old values are read no more
@@ -322,33 +341,50 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     }
     const unsigned char* cols = base + h0.y;
     const unsigned char* vals = base + h0.z;
-    auto use = [&](const FlowQuad<T>& q) {
-      const unsigned i0 = q.c.x & 0xffffu, i1 = q.c.x >> 16, i2 = q.c.y & 0xffffu, i3 = q.c.y >> 16;
-      const V w0 = ring[i0], w1 = ring[i1], w2 = ring[i2], w3 = ring[i3];
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        flow_mac(acc0[r], q.v[0], w0.v[r]);
-        flow_mac(acc1[r], q.v[1], w1.v[r]);
-        flow_mac(acc0[r], q.v[2], w2.v[r]);
-        flow_mac(acc1[r], q.v[3], w3.v[r]);
-      }
-    };
     const int g1 = h1.x & 0xff, g2 = (h1.x >> 8) & 0xff, g4 = (h1.x >> 16) & 0xff;
     int k = 0;
     FlowQuad<T> cur;
     if (g4 > 0) cur = flow_load_quad<T>(cols, vals, l);
+    auto use = [&](T (&s)[4][R]) {
+      FlowQuad<T> nxt = cur;
+      if (k + 1 < g4) nxt = flow_load_quad<T>(cols, vals, (k + 1) * stride + l);
+      const unsigned i0 = cur.c.x & 0xffffu, i1 = cur.c.x >> 16, i2 = cur.c.y & 0xffffu, i3 = cur.c.y >> 16;
+      const V w0 = ring[i0], w1 = ring[i1], w2 = ring[i2], w3 = ring[i3];
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        mac(s[0][r], cur.v[0], w0.v[r]);
+        mac(s[1][r], cur.v[1], w1.v[r]);
+        mac(s[2][r], cur.v[2], w2.v[r]);
+        mac(s[3][r], cur.v[3], w3.v[r]);
+      }
+      cur = nxt;
+      k++;
+    };
     auto run = [&](int end) {
-      for (; k < end; k++) {
-        FlowQuad<T> nxt = cur;
-        if (k + 1 < g4) nxt = flow_load_quad<T>(cols, vals, (k + 1) * stride + l);
-        use(cur);
-        cur = nxt;
+      if constexpr (kFlowSets<T> == 2) {
+        while (k + 1 < end) {
+          use(acc[0]);
+          use(acc[1]);
+        }
+        if (k < end) {  // the sets change places: they are added up alike in the end
+          use(acc[0]);
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+              const T t = acc[0][u][r];
+              acc[0][u][r] = acc[1][u][r];
+              acc[1][u][r] = t;
+            }
+        }
+      } else {
+        while (k < end) use(acc[0]);
       }
     };
-    run(g1);
+    run(min(g1, g4 - 1));
     if (g2 > g1) {
       flow_wait<C::W>(s_prog, h1.z, lane, err, &s_abort);
-      run(g2);
+      run(min(g2, g4 - 1));
     }
     // what the end of the task needs, and the right-hand side of this warp's next task
     const int nch_ = h2.z, noff = h2.w;
@@ -356,13 +392,11 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     T dg = T(1);
     if (UPPER) dg = *(const T*)(base + h0.x + 4 * ((stride + 3) & ~3) + (size_t)l * sizeof(T));
     // operands of the tasks in flight: each is its own flag
-    for (; k < g4; k++) {
-      FlowQuad<T> nxt = cur;
-      if (k + 1 < g4) nxt = flow_load_quad<T>(cols, vals, (k + 1) * stride + l);
+    FlowVal<T, R> w0, w1, w2, w3;
+    auto poll = [&](const FlowQuad<T>& q) {
       const unsigned sz = (unsigned)sizeof(V);
-      const unsigned i0 = ring_at + (cur.c.x & 0xffffu) * sz, i1 = ring_at + (cur.c.x >> 16) * sz,
-                     i2 = ring_at + (cur.c.y & 0xffffu) * sz, i3 = ring_at + (cur.c.y >> 16) * sz;
-      FlowVal<T, R> w0, w1, w2, w3;
+      const unsigned i0 = ring_at + (q.c.x & 0xffffu) * sz, i1 = ring_at + (q.c.x >> 16) * sz,
+                     i2 = ring_at + (q.c.y & 0xffffu) * sz, i3 = ring_at + (q.c.y >> 16) * sz;
       for (int p = 0;; p++) {
         flow_ring_load<T, R>(w0, i0);
         flow_ring_load<T, R>(w1, i1);
@@ -377,19 +411,47 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
           if (*(volatile unsigned*)&s_abort) break;
         }
       }
+    };
+    auto fresh = [&](T (&s)[4][R]) {
+      const FlowQuad<T> nxt = flow_load_quad<T>(cols, vals, (k + 1) * stride + l);
+      poll(cur);
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        flow_mac(acc0[r], cur.v[0], w0.v.v[r]);
-        flow_mac(acc1[r], cur.v[1], w1.v.v[r]);
-        flow_mac(acc0[r], cur.v[2], w2.v.v[r]);
-        flow_mac(acc1[r], cur.v[3], w3.v.v[r]);
+        mac(s[0][r], cur.v[0], w0.v.v[r]);
+        mac(s[1][r], cur.v[1], w1.v.v[r]);
+        mac(s[2][r], cur.v[2], w2.v.v[r]);
+        mac(s[3][r], cur.v[3], w3.v.v[r]);
       }
       cur = nxt;
+      k++;
+    };
+    while (k + 1 < g4) {
+      fresh(acc[0]);
+      if (kFlowSets<T> == 2 && k + 1 < g4) fresh(acc[kFlowSets<T> - 1]);
+    }
+    // the sum of all but the last quad, formed before that is waited for
+    T old[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      T part[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) part[u] = kFlowSets<T> == 2 ? acc[0][u][r] + acc[kFlowSets<T> - 1][u][r] : acc[0][u][r];
+      old[r] = (part[0] + part[2]) + (part[1] + part[3]);
+    }
+    if (g4 > 0) {
+      poll(cur);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        mac(last[0][r], cur.v[0], w0.v.v[r]);
+        mac(last[1][r], cur.v[2], w2.v.v[r]);
+        mac(last[0][r], cur.v[1], w1.v.v[r]);
+        mac(last[1][r], cur.v[3], w3.v.v[r]);
+      }
     }
     FlowVal<T, R> res;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      const T t = b[r] - (acc0[r] + acc1[r]);
+      const T t = b[r] - (old[r] + (last[0][r] + last[1][r]));
       res.v.v[r] = UPPER ? t * dg : t;
     }
     if (on) flow_ring_store<T, R>(ring_at + (unsigned)((h2.y + lane) & (C::ring - 1)) * (unsigned)sizeof(V), res);

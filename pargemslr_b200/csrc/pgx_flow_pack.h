@@ -13,6 +13,16 @@ namespace pgx {
 
 constexpr int kFlowHead = 16;                  // ints of a task header
 constexpr int kFlowMaxQuads = 250;             // quads of one row (a byte each in the header)
+constexpr int kFlowOther = 1 << 30;            // far operand: the set of accumulators the second quad uses
+constexpr int kFlowLast = 1 << 29;             // far operand: one of the row's four newest entries
+constexpr int kFlowIndex = kFlowLast - 1;
+// A row's four newest entries are summed by themselves, the others in
+// kFlowSets sets of four accumulators, successive quads on alternate sets: as
+// many partial sums as the eight lanes a row that summed it before, and no
+// more rounding (the lower pass at 48^3 in FP32 against
+// FP64: 4.1e-8 with eight, 4.4e-8 with four, 4.9e-8 with two).
+template <typename T>
+constexpr int kFlowSets = sizeof(T) <= 8 ? 2 : 1;
 
 // Shared-memory plan of the solve: a ring of the last results (one value per
 // right-hand side and schedule position), then `stages` staging buffers for
@@ -35,7 +45,7 @@ struct FlowPlan {
   static_assert((ring & (ring - 1)) == 0 && vec <= 64, "flow solve: ring");
 };
 constexpr int flow_ring(int vec, bool lng) {
-  return (vec <= 4 ? 8192 : vec <= 16 ? 4096 : 2048) << (lng && vec > 4 && vec < 64 ? 1 : 0);
+  return (vec <= 4 ? 8192 : vec <= 16 ? 4096 : 2048) << (lng && vec < 64 ? 1 : 0);
 }
 // The CTA owns an SM's shared memory.  Twelve warps: with eight the sums of
 // the tasks ahead fall behind the chain (64^3, one lane mixed: 0.39 against
@@ -110,7 +120,7 @@ static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const V
     int f = 0;
     for (int k = rp[i]; k < rp[i + 1]; k++) f += p - pos[cj[k]] > reach;
     len[p] = rp[i + 1] - rp[i];
-    flen[p] = f ? f + 1 : 0;
+    flen[p] = f ? f + 3 : 0;
   }
   auto bytes_of = [&](int a, int e) {
     int mx = 0, mxf = 0;
@@ -171,9 +181,9 @@ static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const V
       nnear[q] = (int)e.size() - f;
       o.nfar += f;
       mx = std::max(mx, nnear[q]);
-      // one more place keeps every entry on the accumulator that its distance
+      // some places more keep every entry on the accumulator that its distance
       // from the row's last entry names
-      mxf = std::max(mxf, f ? f + nnear[q] % 2 : 0);
+      mxf = std::max(mxf, f ? f + nnear[q] % 4 : 0);
     }
     const int quads = (mx + 3) / 4, fq = (mxf + 3) / 4;
     if (quads > kFlowMaxQuads || fq > kFlowMaxQuads) return false;
@@ -224,10 +234,15 @@ static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const V
         const size_t slot = (size_t)(u / 4) * stride + q;
         int* cp = (int*)(b + off_far) + slot * 4 + (u & 3);
         T* vp = (T*)(b + off_far + (size_t)fq * stride * 16) + slot * 4 + (u & 3);
-        const int e = nf ? u - (fq * 4 - nf - nn % 2) : -1;
+        const int e = nf ? u - (fq * 4 - nf - nn % 4) : -1;
         if (e >= 0 && e < nf) {
           const int k = ent[q][e].second;
+          const int back = nn + nf - 1 - e;  // entries of the row after this one
           *cp = upper ? cj[k] : (*up_slot)[cj[k]];
+          if (back < 4)
+            *cp |= kFlowLast;
+          else if (kFlowSets<T> == 2 && (back / 4 + quads + 1) % 2)
+            *cp |= kFlowOther;
           *vp = val(k);
         } else {
           *cp = -1;
@@ -284,7 +299,9 @@ static bool flow_pack(int n, const int* rp, const int* cj, const Val& val, bool 
   std::vector<int> lev(n, 0), pos(n, 0), task_of(n, 0);
   std::vector<FlowPack<T>> part(ncomp);
   std::vector<char> ok(ncomp, 0);
-#pragma omp parallel for schedule(dynamic, 1)
+  // in parallel where that pays: 33,000 entries take 2.6 ms on one thread, and
+  // a team takes 10 ms and more to wake up
+#pragma omp parallel for schedule(dynamic, 1) if (rp[n] > 300000)
   for (int c = 0; c < ncomp; c++)
     ok[c] = flow_pack_comp<T, C>(dom[c], dom[c + 1], rp, cj, val, upper, dinv, up_slot, lev.data(), pos.data(),
                                  task_of.data(), part[c]);
@@ -293,7 +310,7 @@ static bool flow_pack(int n, const int* rp, const int* cj, const Val& val, bool 
     if (!ok[c]) return false;
     bytes += part[c].blob.size();
   }
-  if (bytes / 16 > (size_t)INT_MAX) return false;
+  if (bytes / 16 > (size_t)INT_MAX || n > kFlowIndex) return false;
   o.blob.reserve(bytes);
   o.comp_chunk0.assign(1, 0);
   for (int c = 0; c < ncomp; c++) {

@@ -78,15 +78,18 @@ static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>
       for (int l = 0; l < nr; l++) {
         const int id = ((const int*)(b + h[0]))[l];
         REQ(id >= dom[c] && id < dom[c + 1]);
-        T acc[2] = {T(0), T(0)};
+        T acc[2][4], last[2] = {T(0), T(0)};
+        for (auto& s : acc)
+          for (T& v : s) v = T(0);
         const unsigned char* fv = b + h[13] + (size_t)h[12] * st * 16;
         for (int q = 0; q < h[12]; q++)
           for (int u = 0; u < 4; u++) {
-            const int cc = ((const int*)(b + h[13]))[(q * st + l) * 4 + u];
+            const int raw = ((const int*)(b + h[13]))[(q * st + l) * 4 + u], cc = raw & kFlowIndex;
             const T v = ((const T*)fv)[(q * st + l) * 4 + u];
-            if ((unsigned)cc < (unsigned)n) {
+            if (raw >= 0) {
+              REQ(cc < n);
               REQ(task_of_slot[cc] >= 0 && task_of_slot[cc] + 3 * C::W <= t);
-              acc[u & 1] += v * out[cc];
+              (raw & kFlowLast ? last[u / 2] : acc[raw & kFlowOther ? 1 : 0][u]) += v * out[cc];
             } else {
               REQ(v == T(0));
             }
@@ -103,11 +106,17 @@ static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>
             } else {
               REQ(v == T(0));
             }
-            acc[u & 1] += v * ring[cc];
+            (q == g4 - 1 ? last[u / 2] : acc[kFlowSets<T> == 2 ? q & 1 : 0][u]) += v * ring[cc];
           }
         }
-        acc[0] += acc[1];
-        const T s = (upper ? rhs[h[15] + l] : rhs[id]) - acc[0];
+        T p[4];
+        for (int u = 0; u < 4; u++) (p[u] = acc[0][u]) += acc[1][u];
+        p[0] += p[2];
+        p[1] += p[3];
+        p[0] += p[1];
+        last[0] += last[1];
+        p[0] += last[0];
+        const T s = (upper ? rhs[h[15] + l] : rhs[id]) - p[0];
         res[l] = upper ? s * ((const T*)(b + h[0] + (4 * st + 15) / 16 * 16))[l] : s;
       }
       for (int l = 0; l < nr; l++) {
@@ -135,10 +144,9 @@ struct Tri {
   std::vector<double> va;
 };
 
-template <typename T, int R>
+template <typename T, int R, typename C = FlowCfg<T, R>>
 static int solve(const Tri& L, const Tri& U, const std::vector<double>& dinv, const std::vector<int>& dom, double tol,
                  std::vector<T>* keep) {
-  using C = FlowCfg<T, R>;
   const int n = (int)dinv.size();
   auto lv = [&](int k) { return T(L.va[k]); };
   auto uv = [&](int k) { return T(U.va[k]); };
@@ -253,7 +261,9 @@ int main() {
                       solve<double, 1>(L, U, dinv, cases[q].dom, 4e-15, &kd),
                       solve<double, 4>(L, U, dinv, cases[q].dom, 4e-15, &kd),
                       solve<Wide, 1>(L, U, dinv, cases[q].dom, 4e-15, &kw),
-                      solve<Wide, 4>(L, U, dinv, cases[q].dom, 4e-15, &kw)};
+                      solve<Wide, 4>(L, U, dinv, cases[q].dom, 4e-15, &kw),
+                      solve<float, 1, SysFlowCfg<float>>(L, U, dinv, cases[q].dom, 2e-6, nullptr),
+                      solve<float, 4, FlowCfg<float, 4, true>>(L, U, dinv, cases[q].dom, 2e-6, &kf)};
     for (int r : rc) {
       bad += r == 1;
       packed += r == 0;
