@@ -3940,32 +3940,35 @@ int pgx_gemslr_commit(pgx_handle h) {
   PGX_CUDA(cudaSetDevice(h->device));
   h->extra.clear();
   h->eng.reset();
-  switch (im.precision) {
-    case PGX_PRECISION_MIXED: {
-      auto* e = new Engine<float>();
-      h->eng.reset(e);
-      PGX_TRY(e->commit(im));
-      break;
+  // laying out the factors allocates host memory: no exception may cross the C ABI
+  return guarded("pgx_gemslr_commit", [&]() -> int {
+    switch (im.precision) {
+      case PGX_PRECISION_MIXED: {
+        auto* e = new Engine<float>();
+        h->eng.reset(e);
+        PGX_TRY(e->commit(im));
+        break;
+      }
+      case PGX_PRECISION_COMPLEX_MIXED: {
+        auto* e = new Engine<cf32>();
+        h->eng.reset(e);
+        PGX_TRY(e->commit(im));
+        break;
+      }
+      case PGX_PRECISION_COMPLEX_FP64: {
+        auto* e = new Engine<cf64>();
+        h->eng.reset(e);
+        PGX_TRY(e->commit(im));
+        break;
+      }
+      default: {
+        auto* e = new Engine<double>();
+        h->eng.reset(e);
+        PGX_TRY(e->commit(im));
+      }
     }
-    case PGX_PRECISION_COMPLEX_MIXED: {
-      auto* e = new Engine<cf32>();
-      h->eng.reset(e);
-      PGX_TRY(e->commit(im));
-      break;
-    }
-    case PGX_PRECISION_COMPLEX_FP64: {
-      auto* e = new Engine<cf64>();
-      h->eng.reset(e);
-      PGX_TRY(e->commit(im));
-      break;
-    }
-    default: {
-      auto* e = new Engine<double>();
-      h->eng.reset(e);
-      PGX_TRY(e->commit(im));
-    }
-  }
-  return PGX_SUCCESS;
+    return PGX_SUCCESS;
+  });
 }
 
 // ------------------------------------------------------------ host setup
@@ -4173,14 +4176,16 @@ int pgx_gemslr_set_slots(pgx_handle h, int32_t nslots) {
   if (nslots < 1 || nslots > 256) return fail(PGX_ERROR_INVALID_PARAM, "nslots %d outside [1, 256]", nslots);
   if (h->servers > 0) return fail(PGX_ERROR_FUNCTION_CALL, "slots cannot change while a server is live");
   PGX_CUDA(cudaSetDevice(h->device));
-  while ((int)h->extra.size() > nslots - 1) h->extra.pop_back();
-  while ((int)h->extra.size() < nslots - 1) {
-    std::unique_ptr<EngineBase> e;
-    const int rc = h->eng->make_lanes_clone(h->im, h->lanes, e);
-    if (rc != PGX_SUCCESS) return rc;
-    h->extra.push_back(std::move(e));
-  }
-  return PGX_SUCCESS;
+  return guarded("pgx_gemslr_set_slots", [&]() -> int {
+    while ((int)h->extra.size() > nslots - 1) h->extra.pop_back();
+    while ((int)h->extra.size() < nslots - 1) {
+      std::unique_ptr<EngineBase> e;
+      const int rc = h->eng->make_lanes_clone(h->im, h->lanes, e);
+      if (rc != PGX_SUCCESS) return rc;
+      h->extra.push_back(std::move(e));
+    }
+    return PGX_SUCCESS;
+  });
 }
 
 int pgx_gemslr_set_lanes(pgx_handle h, int32_t lanes) {
@@ -5004,16 +5009,45 @@ int pgx_csr_spmv_device_variant(const pgx_csr* Ad, int32_t variant, double alpha
       return PGX_SUCCESS;
     };
     if (variant == 2) return merge_path();
+    // caller-owned arrays: 128-bit loads only where both are 16-byte aligned
+    // and the nonzeros fill whole 4-entry blocks
+    const bool vec = ((uintptr_t)Ad->colidx % 16 == 0) && ((uintptr_t)Ad->values % 16 == 0) && Ad->nnz % 4 == 0;
     Scratch mem;
-    PGX_TRY(mem.take(sizeof(SpmvPlanDev)));
+    if (mem.take(sizeof(SpmvPlanDev)) != PGX_SUCCESS) {
+      // not a byte of device memory left: the plan is made on the host
+      cudaGetLastError();
+      std::vector<int> rp(Ad->rows + 1);
+      PGX_CUDA(cudaMemcpy(rp.data(), Ad->rowptr, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost));
+      const SpmvPlan p = spmv_plan(Ad->rows, rp.data());
+      if (variant == 0 && p.merge) return merge_path();
+      const int blocks = grid_for(Ad->rows, 256 / p.S, num_sms() * 16);
+#define PGX_SPMV1(SS, VV)                                                                                            \
+  spmv_kernel<double, double, double, double, SS, VV><<<blocks, 256>>>(                                               \
+      Ad->rows, Ad->rowptr, Ad->colidx, Ad->values, x, Ad->cols, alpha, nullptr, nullptr, nullptr, nullptr, 0, 0.0, b, \
+      beta, y, nullptr, nullptr, mk_skip())
+#define PGX_SPMV2(SS) \
+  if (vec)            \
+    PGX_SPMV1(SS, true); \
+  else                \
+    PGX_SPMV1(SS, false)
+      switch (p.S) {
+        case 2: PGX_SPMV2(2); break;
+        case 4: PGX_SPMV2(4); break;
+        case 8: PGX_SPMV2(8); break;
+        case 16: PGX_SPMV2(16); break;
+        default: PGX_SPMV2(32); break;
+      }
+#undef PGX_SPMV2
+#undef PGX_SPMV1
+      PGX_CUDA(cudaGetLastError());
+      PGX_CUDA(cudaDeviceSynchronize());
+      return PGX_SUCCESS;
+    }
     SpmvPlanDev* plan = (SpmvPlanDev*)mem.p;
     PGX_CUDA(cudaMemsetAsync(plan, 0, sizeof(SpmvPlanDev), 0));
     spmv_plan_kernel<<<grid_for(Ad->rows, 1024, num_sms() * 2), 512>>>(Ad->rows, Ad->nnz, Ad->rowptr, plan);
     // the plan is not known here: blocks for eight lanes a row (fewer lanes leave some of them nothing to do)
     const int grid = grid_for(Ad->rows, 32, num_sms() * 16);
-    // caller-owned arrays: 128-bit loads only where both are 16-byte aligned
-    // and the nonzeros fill whole 4-entry blocks
-    const bool vec = ((uintptr_t)Ad->colidx % 16 == 0) && ((uintptr_t)Ad->values % 16 == 0) && Ad->nnz % 4 == 0;
     if (vec)
       spmv_planned_kernel<true><<<grid, 256>>>(plan, variant == 1, Ad->rows, Ad->rowptr, Ad->colidx, Ad->values, x,
                                                Ad->cols, alpha, b, beta, y);

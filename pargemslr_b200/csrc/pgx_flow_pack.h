@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstddef>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -302,9 +303,16 @@ static bool flow_pack(int n, const int* rp, const int* cj, const Val& val, bool 
   // in parallel where that pays: 33,000 entries take 2.6 ms on one thread, and
   // a team takes 10 ms and more to wake up
 #pragma omp parallel for schedule(dynamic, 1) if (rp[n] > 300000)
+  for (int c = 0; c < ncomp; c++) {
+    try {
+      ok[c] = flow_pack_comp<T, C>(dom[c], dom[c + 1], rp, cj, val, upper, dinv, up_slot, lev.data(), pos.data(),
+                                   task_of.data(), part[c]);
+    } catch (const std::bad_alloc&) {
+      ok[c] = 2;  // no exception may leave the parallel region
+    }
+  }
   for (int c = 0; c < ncomp; c++)
-    ok[c] = flow_pack_comp<T, C>(dom[c], dom[c + 1], rp, cj, val, upper, dinv, up_slot, lev.data(), pos.data(),
-                                 task_of.data(), part[c]);
+    if (ok[c] == 2) throw std::bad_alloc();
   size_t bytes = 0;
   for (int c = 0; c < ncomp; c++) {
     if (!ok[c]) return false;
