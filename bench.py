@@ -545,12 +545,12 @@ def run_pgx(args):
     single = {"bytes_per_launch": (lo_bytes + up_bytes) / 2.0, "ms_per_launch": (lo_ms + up_ms) / 2.0}
     single["achieved"] = single["bytes_per_launch"] / (single["ms_per_launch"] * 1e-3) / 1e9
     if args.lanes > 1:
-        kname = ("trsv_pipe_kernel (level-0 ILU L and U passes merged over %d lanes, mean; one CTA per "
+        kname = ("trsv_flow_kernel (level-0 ILU L and U passes merged over %d lanes, mean; one CTA per "
                  "subdomain)" % args.lanes)
         tri_bytes = (blo_bytes + bup_bytes) / 2.0
         tri_ms = (blo_ms + bup_ms) / 2.0
     else:
-        kname = "trsv_pipe_kernel (level-0 ILU L and U passes, mean; one CTA per subdomain)"
+        kname = "trsv_flow_kernel (level-0 ILU L and U passes, mean; one CTA per subdomain)"
         tri_bytes, tri_ms = single["bytes_per_launch"], single["ms_per_launch"]
     achieved = tri_bytes / (tri_ms * 1e-3) / 1e9
     traffic = ncu_traffic(args.lanes)
