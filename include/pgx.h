@@ -383,7 +383,7 @@ int pgx_pool_destroy(pgx_pool pool);
  *     sixteenth; stride 1 is the whole batch) from x0 = 0 into the object's
  *     own vectors, by coordinate descent over the CTA shape (256 threads x 2
  *     per SM, 512 x 1, 512 x 2, 1024 x 1), then the SpMV lanes per row (2, 4,
- *     8), then the levels the triangular passes fetch ahead (2, 3); it keeps
+ *     8), then the levels the packed triangular passes fetch ahead (2, 3); it keeps
  *     the fastest and returns its device time.  pgx_systems_tune_table returns
  *     the candidates tried, five doubles each (threads, CTAs per SM, lanes,
  *     depth, ms).
@@ -419,16 +419,17 @@ int pgx_gemslr_precond_apply(pgx_handle handle, double *z, const double *v, int3
  * block of the solve: which 0 = lower triangular pass of `level`, 1 = upper
  * triangular pass of `level`, 2 = outer CSR SpMV, 3 / 4 = the lower / upper
  * pass of `level` merged over the lanes of a multi-lane slot (vectors counted
- * once per lane, the factor once).  Algorithmic bytes count
- * every operand once: nnz*(value+index) + row pointers + schedule + vectors
- * in and out. */
+ * once per lane, the factor once).  A level whose factors are solved by one
+ * product (pgx_gemslr_describe names it) reports the product as its lower
+ * pass.  Algorithmic bytes count every operand once: nnz*(value+index) + row
+ * pointers + schedule + vectors in and out. */
 int pgx_gemslr_kernel_stats(pgx_handle handle, int32_t which, int32_t level, int32_t reps, double *avg_ms,
                             double *bytes);
 
 /* A text description of slot `slot` of a committed handle (0 = the handle's
  * own slot), one line per structure: for every level the kernel and layout
- * of the L and U passes (per-subdomain pipeline, segmented or level-set;
- * lanes per row, dependency levels, chunks) and the SpMV variant of A, E_l,
+ * of the L and U passes (per-subdomain dataflow, one product of the inverses,
+ * segmented or level-set; dependency levels, tasks, chunks) and the SpMV variant of A, E_l,
  * F_l and C_0 (lanes per row or merge path); for a multi-lane slot its
  * merged layouts.  Plays the part of the reference's setup report
  * (GemslrClass print level).  *length receives the text's length; at most
