@@ -176,6 +176,7 @@ template <typename C>
 struct FlowShared {
   unsigned long long full[C::stages];  // a chunk has landed
   unsigned prog[C::W], freed[C::stages], abort;
+  unsigned issued;  // chunks whose copies are issued
 };
 
 // One pass over subdomain `comp`, whose chunks are a.chunk[c0 .. c0 + nch):
@@ -194,13 +195,14 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
   V* ring = (V*)smem_raw;
   unsigned char* stage0 = smem_raw + C::ring_bytes;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) {
+  if (tid == 0) {
     // a wait of an earlier pass gave up: the solve reports the timeout, and the passes after it do no work
     s_abort = (*(volatile int*)err & (kErrTimeout | kErrStage)) != 0;
     for (int s = 0; s < D; s++) {
       mbar_init(&s_full[s], 1);
       s_freed[s] = 0;
     }
+    sh.issued = 0;
     mbar_fence_init();
   }
   if (tid < C::W) s_prog[tid] = 0;
@@ -243,6 +245,7 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
               mbar_arrive_expect_tx(&s_full[s], (unsigned)m.y * 16u);
               bulk_g2s(stage0 + (size_t)s * C::stage_bytes, a.blob + (size_t)m.x * 16, (unsigned)m.y * 16u, &s_full[s]);
               c++;
+              flow_st(&sh.issued, (unsigned)c);
             }
           }
         }
@@ -259,8 +262,17 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
 #pragma unroll
   for (int r = 0; r < R; r++) b[r] = T(0);
   const unsigned ring_at = smem_u32(smem_raw);
-  unsigned mine = 0;  // tasks this warp has done
+  unsigned mine = 0;    // tasks this warp has done
+  unsigned issued = 0;  // chunks this lane knows to be issued
   while (ch >= 0) {
+    for (int k = 0; !flow_issued(issued, ch) && !*(volatile unsigned*)&s_abort; k++) {
+      issued = flow_ld(&sh.issued);
+      if (k >= kFlowPolls) {
+        atomicOr(err, kErrStage);
+        *(volatile unsigned*)&s_abort = 1u;
+      }
+    }
+    __syncwarp();
     if (*(volatile unsigned*)&s_abort) break;
     const int st = ch % D;
     if (!mbar_wait(&s_full[st], (unsigned)((ch / D) & 1), err)) {
@@ -473,7 +485,8 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     T bn[R];
 #pragma unroll
     for (int r = 0; r < R; r++) bn[r] = T(0);
-    if (nch_ >= 0 && mbar_try_wait(&s_full[nch_ % D], (unsigned)((nch_ / D) & 1))) {
+    if (nch_ >= 0 && !flow_issued(issued, nch_)) issued = flow_ld(&sh.issued);
+    if (nch_ >= 0 && flow_issued(issued, nch_) && mbar_try_wait(&s_full[nch_ % D], (unsigned)((nch_ / D) & 1))) {
       const unsigned char* nbase = stage0 + (size_t)(nch_ % D) * C::stage_bytes;
       const int nr2 = *(const int*)(nbase + noff + 12) & 0xff;
       const int l2 = lane < nr2 ? lane : 0;

@@ -25,6 +25,17 @@ constexpr int kFlowIndex = kFlowLast - 1;
 template <typename T>
 constexpr int kFlowSets = sizeof(T) <= 8 ? 2 : 1;
 
+// Whether a warp may test the barrier of chunk `chunk`, with `issued` chunks
+// issued so far.  Chunk c uses the stage and the barrier of chunk c - stages
+// again, and the test is by parity: while that older chunk is on its way the
+// barrier looks as if c had landed, and copies land in any order.  A chunk
+// is issued only after the older one is consumed, so once it is issued the
+// parity says what it should.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool flow_issued(unsigned issued, int chunk) { return issued > (unsigned)chunk; }
+
 // Shared-memory plan of the solve: a ring of the last results (one value per
 // right-hand side and schedule position), then `stages` staging buffers for
 // the factor.
@@ -40,8 +51,8 @@ struct FlowPlan {
   static constexpr int ahead = 32 * (W + 2);           // a task clears the ring slots of the rows this far ahead
   static constexpr int reach = ring - ahead - 32 * W;  // operands at most this old are in the ring
   static constexpr size_t bytes = ring_bytes + (size_t)stages * stage_bytes;
-  // a warp looks one task of its own ahead, at most W chunks: with fewer
-  // stages the barrier it tests could belong to the chunk two uses back
+  // a warp looks one task of its own ahead, at most W chunks: with at least W
+  // stages that chunk can be on its way while the warp is still in its own
   static_assert(stages >= W && W >= 2 && ring >= ahead + 32 * (4 * W + 1), "flow solve: shared memory");
   static_assert((ring & (ring - 1)) == 0 && vec <= 64, "flow solve: ring");
 };

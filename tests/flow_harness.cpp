@@ -29,13 +29,75 @@ struct Wide {  // a complex value
   bool operator==(const Wide& o) const { return x == o.x && y == o.y; }
 };
 
-// the kernel's walk, task by task in schedule order; `order_of` receives the
-// entries of each row in the order and on the accumulator they are summed
+struct Task {  // what a task waits for: its chunk, its progress limit and its sources
+  int chunk, next_chunk, lim;
+  std::vector<int> src;
+};
+
+// One subdomain's pass with copies that land in any order among those in
+// flight.  A copy lands only when nothing else can move (`newest`: the last
+// one issued first, else any), which is as late as it can be.  Every stage
+// that a barrier test lets a warp read must hold the chunk that was meant.
+template <typename C>
+static bool land(const std::vector<Task>& ts, const int* chunk, int nch, std::mt19937& g, bool newest) {
+  constexpr int D = C::stages, W = C::W;
+  const int nt = (int)ts.size();
+  std::vector<int> freed(D, 0), tot(D, 0), phases(D, 0), holds(D, -1), flight;
+  std::vector<char> done(nt, 0), in(W, 0);
+  std::vector<int> at(W);
+  for (int w = 0; w < W; w++) at[w] = w;
+  int issued = 0, below = 0;  // chunks issued; every task below `below` is done
+  auto full = [&](int ch) { return flow_issued((unsigned)issued, ch) && (phases[ch % D] & 1) != ((ch / D) & 1); };
+  for (;;) {
+    bool moved = false;
+    for (; issued < nch && (issued < D || freed[issued % D] >= tot[issued % D]); issued++) {
+      tot[issued % D] += chunk[4 * issued + 2];
+      holds[issued % D] = -1;
+      flight.push_back(issued);
+      moved = true;
+    }
+    for (int w = 0; w < W; w++) {
+      const int t = at[w];
+      if (t >= nt) continue;
+      const Task& k = ts[t];
+      if (!in[w]) {
+        if (!full(k.chunk)) continue;
+        REQ(holds[k.chunk % D] == k.chunk);
+        in[w] = 1;
+        moved = true;
+      }
+      bool ready = below >= k.lim;
+      for (int s : k.src) ready = ready && done[s];
+      if (!ready) continue;
+      done[t] = 1;
+      while (below < nt && done[below]) below++;
+      freed[k.chunk % D]++;
+      in[w] = 0;
+      at[w] += W;
+      REQ((at[w] < nt ? ts[at[w]].chunk : -1) == k.next_chunk);
+      if (k.next_chunk >= 0 && full(k.next_chunk)) REQ(holds[k.next_chunk % D] == k.next_chunk);
+      moved = true;
+    }
+    if (moved) continue;
+    if (flight.empty()) break;
+    const size_t q = newest ? flight.size() - 1 : g() % flight.size();
+    holds[flight[q] % D] = flight[q];
+    phases[flight[q] % D]++;
+    flight.erase(flight.begin() + (long)q);
+  }
+  REQ(below == nt && issued == nch);
+  return true;
+}
+
+// the kernel's walk, task by task in schedule order, then the same with
+// copies that land out of order
 template <typename T, typename C>
 static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>& dom, const std::vector<T>& rhs,
                  std::vector<T>& out) {
   out.assign(n, T(0));
+  std::mt19937 gl(9);
   for (int c = 0; c < p.ncomp; c++) {
+    std::vector<Task> tasks;
     const int c0 = p.comp_chunk0[c], nch = p.comp_chunk0[c + 1] - c0;
     REQ((nch == 0) == (dom[c] == dom[c + 1]));
     std::vector<int> wch(C::W), woff(C::W), cnt(nch, 0), task_of_slot(n, -1);
@@ -74,6 +136,11 @@ static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>
         owner[s] = -1;
         read_by[s] = -1000;
       }
+      tasks.push_back({ch, h[10], g2 > g1 ? h[6] : h[5], {}});
+      auto source = [&](int s) {
+        auto& v = tasks.back().src;
+        if (std::find(v.begin(), v.end(), s) == v.end()) v.push_back(s);
+      };
       std::vector<T> res(nr);
       for (int l = 0; l < nr; l++) {
         const int id = ((const int*)(b + h[0]))[l];
@@ -89,6 +156,7 @@ static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>
             if (raw >= 0) {
               REQ(cc < n);
               REQ(task_of_slot[cc] >= 0 && task_of_slot[cc] + 3 * C::W <= t);
+              source(task_of_slot[cc]);
               (raw & kFlowLast ? last[u / 2] : acc[raw & kFlowOther ? 1 : 0][u]) += v * out[cc];
             } else {
               REQ(v == T(0));
@@ -102,6 +170,7 @@ static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>
             REQ(cc <= C::ring);
             if (cc < C::ring) {
               REQ(owner[cc] >= 0 && owner[cc] < before);
+              source(owner[cc]);
               read_by[cc] = t;
             } else {
               REQ(v == T(0));
@@ -135,6 +204,8 @@ static bool walk(const FlowPack<T>& p, int n, bool upper, const std::vector<int>
     }
     REQ(rows == dom[c + 1] - dom[c]);
     for (int k = 0; k < nch; k++) REQ(cnt[k] == p.chunk[4 * (size_t)(c0 + k) + 2]);
+    for (int k = 0; k < 3; k++)
+      if (nch > 0) REQ((land<C>(tasks, &p.chunk[4 * (size_t)c0], nch, gl, k == 0)));
   }
   return true;
 }
@@ -232,6 +303,29 @@ static void make(const std::vector<int>& dom, int deg, int back, int longrow, un
     }
 }
 
+// a factor pair on an nx x ny x nz grid: the neighbours within `reach` in every direction that come before (after) a
+// row, as a factor with much fill has them
+static void grid(int nx, int ny, int nz, int reach, unsigned seed, Tri& L, Tri& U, std::vector<double>& dinv) {
+  std::mt19937 g(seed);
+  std::uniform_real_distribution<double> d(-1, 1);
+  for (int i = 0; i < nx * ny * nz; i++) {
+    const int x = i % nx, y = i / nx % ny, z = i / (nx * ny);
+    for (int up = 0; up < 2; up++) {
+      Tri& M = up ? U : L;
+      for (int c = std::max(0, z - 1); c <= std::min(nz - 1, z + 1); c++)
+        for (int b = std::max(0, y - reach); b <= std::min(ny - 1, y + reach); b++)
+          for (int a = std::max(0, x - reach); a <= std::min(nx - 1, x + reach); a++) {
+            const int j = (c * ny + b) * nx + a;
+            if (up ? j <= i : j >= i) continue;
+            M.cj.push_back(j);
+            M.va.push_back((float)(d(g) / 60));
+          }
+      M.rp.push_back((int)M.cj.size());
+    }
+    dinv.push_back((float)(1.0 + 0.2 * d(g)));
+  }
+}
+
 int main() {
   struct Case {
     std::vector<int> dom;
@@ -268,6 +362,27 @@ int main() {
       bad += r == 1;
       packed += r == 0;
       if (r == 1) std::printf("case %zu\n", q);
+    }
+  }
+  // chunks of few tasks: some 21 entries a row, under every layout
+  {
+    Tri L, U;
+    std::vector<double> dinv;
+    grid(48, 48, 16, 2, 5, L, U, dinv);
+    const std::vector<int> dom = {0, (int)dinv.size()};
+    const int rc[] = {solve<float, 1>(L, U, dinv, dom, 2e-6, nullptr),
+                      solve<float, 4>(L, U, dinv, dom, 2e-6, nullptr),
+                      solve<double, 1>(L, U, dinv, dom, 4e-15, nullptr),
+                      solve<double, 4>(L, U, dinv, dom, 4e-15, nullptr),
+                      solve<Wide, 1>(L, U, dinv, dom, 4e-15, nullptr),
+                      solve<Wide, 4>(L, U, dinv, dom, 4e-15, nullptr),
+                      solve<float, 1, FlowCfg<float, 1, true>>(L, U, dinv, dom, 2e-6, nullptr),
+                      solve<double, 4, FlowCfg<double, 4, true>>(L, U, dinv, dom, 4e-15, nullptr),
+                      solve<float, 1, SysFlowCfg<float>>(L, U, dinv, dom, 2e-6, nullptr),
+                      solve<double, 1, SysFlowCfg<double>>(L, U, dinv, dom, 4e-15, nullptr)};
+    for (const int& r : rc) {
+      bad += r != 0;
+      if (r) std::printf("grid: layout %d, result %d\n", (int)(&r - rc), r);
     }
   }
   // what the kernel does not take is refused: coupled subdomains, a row that no task can hold
