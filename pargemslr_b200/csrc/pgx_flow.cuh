@@ -60,7 +60,10 @@ __device__ __forceinline__ void flow_wait(unsigned* prog, int lim, int lane, int
   const unsigned need = lane < W && lim > lane ? (unsigned)(lim - lane + W - 1) / W : 0u;
   for (int k = 0;; k++) {
     const unsigned v = lane < W ? flow_ld(&prog[lane]) : 0u;
-    if (__all_sync(0xffffffffu, v >= need)) return;
+    if (__all_sync(0xffffffffu, v >= need)) {
+      __syncwarp();  // a vote orders no memory: the lanes that acquired hand over to the others here
+      return;
+    }
     if ((k & 255) == 255) {
       if (k >= kFlowPolls) {
         atomicOr(err, kErrStage);

@@ -83,6 +83,45 @@ def test_pass_pair(name, cplx, precision):
     assert np.linalg.norm(z - ref) <= tol * np.linalg.norm(ref)
 
 
+def _one_level(dom, L, U, dinv):
+    n = dom[-1]
+    eye = (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n, dinv.dtype), n, n)
+    lv = LevelStructures(ncomp=len(dom) - 1, dom_ptr=np.array(dom, np.int32), L=L, U=U, dinv=dinv, B=eye)
+    return GemslrStructures(n=n, A=eye, pperm=np.arange(n, dtype=np.int32), qperm=None,
+                            lev_ptr=np.array([0, n], np.int32), levels=[lv], inner_enable=0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+@pytest.mark.parametrize("name", [k for k in CASES if k not in ("one row", "diagonal")])
+def test_lanes_repeat_the_single_lane(name, cplx, precision):
+    """The same solves through slots of one, two and four lanes: the same results bit for bit, on every pass."""
+    from pargemslr_b200 import params as P
+    from pargemslr_b200.handle import GemslrHandle
+    dom, deg, back, longrow = CASES[name]
+    if name in ("a task and a row", "chains"):
+        deg, back = 3, 2  # one row a level: well above the depth of one product
+    L, U, dinv = _factors(dom, deg, back, len(name), cplx, longrow)
+    n = dom[-1]
+    rng = np.random.default_rng(2)
+    B = rng.standard_normal((4, n)) + (1j * rng.standard_normal((4, n)) if cplx else 0.0)
+    p = P.workload_params("lap2d_256")
+    h = GemslrHandle(_one_level(dom, L, U, dinv), precision=precision)
+    try:
+        assert "dataflow" in h.describe()
+        want = [h.solve(b, params=p)[0] for b in B]
+        for lanes in (2, 4):
+            h.set_lanes(lanes)
+            h.set_slots(1 + 4 // lanes)
+            for _ in range(2):
+                X, R = h.solve_batch(B, params=p)
+                assert all(r["status"] == 0 for r in R)
+                for k in range(4):
+                    np.testing.assert_array_equal(X[k], want[k])
+    finally:
+        h.close()
+
+
 @pytest.mark.parametrize("levels", [2, 7, 8, 9])
 @pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
 def test_shallow_factors(levels, cplx):
