@@ -215,6 +215,10 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     for (int i = tid; i < words + (int)sizeof(V) / 4; i += blockDim.x)
       w[i] = i >= words ? 0u : kFlowWide<T> ? kFlowS64 : kFlowS32;
   }
+  // the stages may hold what this thread wrote before the pass (the systems
+  // kernel's packed passes use the same buffer); a CTA barrier alone does not
+  // order that before the bulk copies
+  proxy_fence_smem();
   __syncthreads();
   if (s_abort || warp > C::W) return;
   if (warp == C::W) {
@@ -242,6 +246,7 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
                 }
                 __nanosleep(32);
               }
+              proxy_fence_smem();  // the reads of the stage's last use, acquired above, before the copy over them
             }
             if (ok) {
               tot[s] += m.z;

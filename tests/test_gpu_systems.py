@@ -178,3 +178,54 @@ def test_reference_setups_in_one_launch_match_the_reference(precision):
     sb.close()
     for h in handles:
         h.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_packed_and_dataflow_passes_take_turns_in_one_buffer(precision):
+    """Two levels on either side of the depth from which a pass runs by dataflow: 12,000 rows three levels deep
+    (packed passes, whose ring of solved values reaches over the staging buffers of the other kind) and 700 rows one
+    level each.  The passes alternate in one CTA's shared memory; every solve gives the same bits, and those of the
+    handle's own solve to rounding."""
+    import scipy.sparse as sp
+
+    from pargemslr_b200.handle import GemslrHandle
+    from pargemslr_b200.structures import GemslrStructures, LevelStructures
+    from pargemslr_b200.systems import SystemsBatch
+    rng = np.random.default_rng(6)
+    n0, n1, step = 12000, 700, 4000
+    shallow = sp.csr_matrix((rng.uniform(-0.4, 0.4, n0 - step), (np.arange(step, n0), np.arange(n0 - step))),
+                            shape=(n0, n0))
+    deep = sp.diags([rng.uniform(-0.3, 0.3, n1 - k) for k in (1, 2, 7)], [-1, -2, -7], format="csr")
+
+    def tup(m):
+        m = sp.csr_matrix(m)
+        m.sort_indices()
+        return m.indptr.astype(np.int32), m.indices.astype(np.int32), m.data.astype(np.float64), *m.shape
+
+    levels, blocks = [], []
+    for low, n in ((shallow, n0), (deep, n1)):
+        up, dinv = sp.csr_matrix(low.T) * 0.8, 1.0 + 0.2 * rng.uniform(-1, 1, n)
+        B = (sp.identity(n) + low) @ (sp.diags(1.0 / dinv) + up)
+        levels.append(LevelStructures(ncomp=1, dom_ptr=np.array([0, n], np.int32), L=tup(low), U=tup(up), dinv=dinv,
+                                      B=tup(B)))
+        blocks.append(B)
+    E = sp.random(n1, n0, 2e-4, random_state=3, format="csr") * 0.1
+    F = sp.csr_matrix(E.T)
+    levels[0].E, levels[0].F = tup(E), tup(F)
+    A = tup(sp.bmat([[blocks[0], F], [E, blocks[1]]]))
+    st = GemslrStructures(n=n0 + n1, A=A, pperm=np.arange(n0 + n1, dtype=np.int32), qperm=None,
+                          lev_ptr=np.array([0, n0, n0 + n1], np.int32), levels=levels, inner_enable=0)
+    p = _convdiff_params()
+    h = GemslrHandle(st, precision=precision)
+    sb = SystemsBatch([h])
+    b = problems.spmv(A[:3], rng.standard_normal(n0 + n1))
+    first, R = sb.solve([b], params=p)
+    assert R[0]["status"] == 0 and R[0]["true_rel_res"] <= 1e-8
+    for _ in range(4):
+        X, _ = sb.solve([b], params=p)
+        np.testing.assert_array_equal(X[0], first[0])
+    xs, rs = h.solve(b, params=p)
+    assert abs(rs["iters"] - R[0]["iters"]) <= 1
+    assert np.linalg.norm(first[0] - xs) <= 1e-6 * np.linalg.norm(xs)
+    sb.close()
+    h.close()
