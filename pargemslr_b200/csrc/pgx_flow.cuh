@@ -54,7 +54,8 @@ __device__ __forceinline__ void flow_st(unsigned* p, unsigned v) {
 __device__ __forceinline__ void flow_add(unsigned* p) {
   asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(p)) : "memory");
 }
-// until every task below `lim` is done (bounded); task t belongs to warp t % W, prog[w] counts warp w's done tasks
+// until every task below `lim` is done (bounded); task t belongs to warp t % W, prog[w] counts warp w's done tasks.
+// A warp gives up as a whole: its lanes meet in votes and warp barriers again.
 template <int W>
 __device__ __forceinline__ void flow_wait(unsigned* prog, int lim, int lane, int* err, unsigned* abort) {
   const unsigned need = lane < W && lim > lane ? (unsigned)(lim - lane + W - 1) / W : 0u;
@@ -69,7 +70,7 @@ __device__ __forceinline__ void flow_wait(unsigned* prog, int lim, int lane, int
         atomicOr(err, kErrStage);
         *(volatile unsigned*)abort = 1u;
       }
-      if (*(volatile unsigned*)abort) return;
+      if (__any_sync(0xffffffffu, *(volatile unsigned*)abort != 0)) return;
     }
   }
 }
@@ -280,10 +281,9 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
         *(volatile unsigned*)&s_abort = 1u;
       }
     }
-    __syncwarp();
-    if (*(volatile unsigned*)&s_abort) break;
+    if (__any_sync(0xffffffffu, *(volatile unsigned*)&s_abort != 0)) break;
     const int st = ch % D;
-    if (!mbar_wait(&s_full[st], (unsigned)((ch / D) & 1), err)) {
+    if (!__all_sync(0xffffffffu, mbar_wait(&s_full[st], (unsigned)((ch / D) & 1), err))) {
       s_abort = 1;
       break;
     }
