@@ -967,19 +967,23 @@ struct Engine : EngineBase {
   // the level recursion of one preconditioner application (rt -> xt, the
   // slot's own vectors) as a graph, from the handle's second application on
   cudaGraphExec_t apply_exec = nullptr;
-  bool applied = false;
+  bool applied = false, apply_direct = false;  // apply_direct: no graph could be made
 
-  void drop_graph() {
+  void drop_cycle() {
     if (cycle_exec) cudaGraphExecDestroy(cycle_exec);
-    if (apply_exec) cudaGraphExecDestroy(apply_exec);
-    cycle_exec = apply_exec = nullptr;
-    applied = false;
+    cycle_exec = nullptr;
     g_kdim = -1;
+  }
+  void drop_graphs() {
+    drop_cycle();
+    if (apply_exec) cudaGraphExecDestroy(apply_exec);
+    apply_exec = nullptr;
+    applied = apply_direct = false;
   }
 
   ~Engine() override {
     if (stream) cudaStreamSynchronize(stream);
-    drop_graph();
+    drop_graphs();
     ar.release();
     wk.release();
     krylov.release();
@@ -1447,7 +1451,7 @@ struct Engine : EngineBase {
   int ensure_krylov(int kdim) {
     if (kdim <= kdim_alloc) return PGX_SUCCESS;
     PGX_CUDA(cudaStreamSynchronize(stream));
-    drop_graph();
+    drop_cycle();
     krylov.release();
     PGX_TRY(krylov.zeros(&V, (size_t)n * (kdim + 1), stream));
     PGX_TRY(krylov.zeros(&Z, (size_t)n * (kdim + 1), stream));
@@ -1858,6 +1862,24 @@ struct Engine : EngineBase {
     return PGX_SUCCESS;
   }
 
+  void capture_levels() {
+    apply_direct = true;
+    if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      levels(mk_skip());
+      cudaGraph_t g = nullptr;
+      if (cudaStreamEndCapture(stream, &g) == cudaSuccess) {
+        if (cudaGraphInstantiate(&apply_exec, g, 0) == cudaSuccess && cudaGraphUpload(apply_exec, stream) == cudaSuccess)
+          apply_direct = false;
+        cudaGraphDestroy(g);
+      }
+    }
+    if (apply_direct) {
+      if (apply_exec) cudaGraphExecDestroy(apply_exec);
+      apply_exec = nullptr;
+      cudaGetLastError();
+    }
+  }
+
   int apply(double* z_, const double* v_, int location) override {
     F* z = (F*)z_;
     const F* v = (const F*)v_;
@@ -1871,20 +1893,10 @@ struct Engine : EngineBase {
     // One application launches a hundred kernels of a few microseconds each;
     // as a graph they follow one another without the host (B200: 64^2 FP64 904
     // -> 739 us, 48^3 mixed 3.89 -> 3.65 ms).  The first application runs
-    // without it: a handle applied once does not pay for the capture.
-    if (applied && !apply_exec) {
-      cudaGraph_t g = nullptr;
-      PGX_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      levels(mk_skip());
-      cudaError_t ce = cudaStreamEndCapture(stream, &g);
-      if (ce != cudaSuccess) return fail(PGX_ERROR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
-      ce = cudaGraphInstantiate(&apply_exec, g, 0);
-      cudaGraphDestroy(g);
-      if (ce != cudaSuccess) {
-        apply_exec = nullptr;
-        return fail(PGX_ERROR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
-      }
-    }
+    // without it: a handle applied once does not pay for the capture.  Where
+    // no graph can be made (no device memory left, say) the kernels go on
+    // being launched one by one.
+    if (applied && !apply_exec && !apply_direct) capture_levels();
     applied = true;
     PGX_CUDA(cudaMemsetAsync(err, 0, sizeof(int), stream));
     precond<F>(vin, nullptr, zout, mk_skip(), apply_exec);
@@ -1946,7 +1958,7 @@ struct Engine : EngineBase {
     PGX_TRY(begin_prologue(x, b, location, kdim, maxits, tol, atol, &xd, &bd, prechecked));
     s_max_cycles = maxits > 0 ? maxits / kdim + 2 : 0;
     if (s_max_cycles > 0 && (!cycle_exec || g_kdim != kdim || g_x != xd || g_b != bd)) {
-      drop_graph();
+      drop_cycle();
       cudaGraph_t g = nullptr;
       PGX_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
       enqueue_cycle(kdim, xd, bd);
@@ -2215,7 +2227,7 @@ struct Engine : EngineBase {
   void set_wait_limit(int polls) override {
     if (stream) cudaStreamSynchronize(stream);
     spin_limit = polls;
-    drop_graph();
+    drop_graphs();
   }
 
   // batched factor layouts shared by this handle's multi-lane slots, by lane count
