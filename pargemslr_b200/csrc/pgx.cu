@@ -584,9 +584,27 @@ static int upload_tri_seg(Arena& ar, const HostCsr& h, bool upper, const std::ve
   return PGX_SUCCESS;
 }
 
+// Operands that left the ring ("far") cost one SM about 1.3 ns each, and the
+// pass of a subdomain runs on one SM.  Where most operands are far (levels of
+// hundreds of unrelated rows) a large subdomain is better off with the
+// segmented kernel, which spreads it over several.  Random matrices, 32
+// entries a row, mixed, on a B200; dataflow against segmented: level-0 passes
+// (lower + upper), one solve, 24 solves at once on one-lane and on four-lane slots, ms:
+//    20k rows (  9k far)  0.21 / 0.75    1.65 / 4.35    5.0 / 13.1     7.6 / 19.4
+//    60k      (1.26M)     1.42 / 1.33    7.9  / 7.5    14.5 / 13.6    41.9 / 32.2
+//    80k      (1.86M)     2.09 / 1.61   11.3  / 9.0    19.6 / 18.0    58   / 39.6
+//   200k      (5.56M)     6.5  / 2.55   38.5  / 14.2   44.2 / 34.9   156   / 62.1
+//   500k      (14.9M)    20.4  / 3.36  104    / 18.4  114   / 52.1   419   / 87.1
+// The line is a million in one pass of one subdomain, a little above where the
+// two are equal (at 80k rows the upper factor meets it with the longer ring:
+// one solve 10.5 ms).  It is drawn by the one-lane layout: lanes go where
+// their handle goes.
+constexpr long long kFlowMostFar = 1000000;
+
 // The per-subdomain schedule of trsv_flow_kernel for R right-hand sides.
 // Returns PGX_ERROR_INVALID_PARAM (and builds nothing) when the factor does
-// not suit the kernel (it couples two subdomains, or a row is too long).
+// not suit the kernel (it couples two subdomains, a row is too long, or most
+// operands are far).
 template <typename T, int R>
 static int upload_tri_flow(Arena& ar, const HostCsr& h, bool upper, const std::vector<int>& dom, DTri<T>& d,
                            cudaStream_t s, const std::vector<double>* dinv, std::vector<int>* slot_of_row,
@@ -600,7 +618,8 @@ static int upload_tri_flow(Arena& ar, const HostCsr& h, bool upper, const std::v
   FlowPack<T> pk;
   auto val = [&](int k) { return hval<T>(h.va.data(), (size_t)k); };
   auto diag = [&](int i) { return hval<T>(dinv->data(), (size_t)i); };
-  const bool fits = flow_pack<T, C>(n, h.rp.data(), h.cj.data(), val, upper, cuts, &diag, upper_slot_of_row, pk);
+  const long long most = R == 1 ? kFlowMostFar : LLONG_MAX;
+  const bool fits = flow_pack<T, C>(n, h.rp.data(), h.cj.data(), val, upper, cuts, &diag, upper_slot_of_row, pk, most);
   // Operands that left the ring are read back from global memory.  When they
   // are more than a hundredth of the entries, a ring twice as long with fewer
   // warps is the better trade.  128^3, lower pass on a B200: four lanes mixed,
@@ -612,7 +631,7 @@ static int upload_tri_flow(Arena& ar, const HostCsr& h, bool upper, const std::v
     if (!fits || pk.nfar * 100 > h.nnz()) {
       FlowPack<T> lk;
       if (flow_pack<T, FlowCfg<T, R, true>>(n, h.rp.data(), h.cj.data(), val, upper, cuts, &diag, upper_slot_of_row,
-                                            lk) &&
+                                            lk, most) &&
           (!fits || 2 * lk.nfar < pk.nfar)) {
         d.flow_long = true;
         std::swap(pk, lk);

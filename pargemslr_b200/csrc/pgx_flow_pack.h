@@ -98,7 +98,8 @@ struct FlowPack {
 // one subdomain, rows [r0, r1)
 template <typename T, typename C, typename Val, typename Diag>
 static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const Val& val, bool upper, const Diag* dinv,
-                           const std::vector<int>* up_slot, int* lev, int* pos, int* task_of, FlowPack<T>& o) {
+                           const std::vector<int>* up_slot, int* lev, int* pos, int* task_of, long long most_far,
+                           FlowPack<T>& o) {
   const int m = r1 - r0;
   auto align16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
   // dependency levels and the schedule: rows by level, then by index
@@ -122,6 +123,10 @@ static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const V
     for (int i = r0; i < r1; i++) order[cur[lev[i]]++] = i;
   }
   for (int p = 0; p < m; p++) pos[order[p]] = p;
+  long long far = 0;
+  for (int i = r0; i < r1; i++)
+    for (int k = rp[i]; k < rp[i + 1]; k++) far += pos[i] - pos[cj[k]] > C::reach;
+  if (far > most_far && 2 * far > rp[r1] - rp[r0]) return false;
   // tasks: at most 32 rows of one level.  The bound of a task's image holds
   // under every lane count, so all of them cut the same tasks (and sum every
   // row in the same order).
@@ -300,11 +305,13 @@ static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const V
 }
 
 // Returns false when the factor does not suit the kernel: it couples two
-// subdomains, a row is too long, or an operand is too old for the ring yet
-// too new to be read back.
+// subdomains, a row is too long, an operand is too old for the ring yet too
+// new to be read back, or most operands of a subdomain, and more than
+// `most_far`, are that old.
 template <typename T, typename C, typename Val, typename Diag>
 static bool flow_pack(int n, const int* rp, const int* cj, const Val& val, bool upper, const std::vector<int>& dom,
-                      const Diag* dinv, const std::vector<int>* up_slot, FlowPack<T>& o) {
+                      const Diag* dinv, const std::vector<int>* up_slot, FlowPack<T>& o,
+                      long long most_far = LLONG_MAX) {
   const int ncomp = (int)dom.size() - 1;
   o = FlowPack<T>();
   o.ncomp = ncomp;
@@ -317,7 +324,7 @@ static bool flow_pack(int n, const int* rp, const int* cj, const Val& val, bool 
   for (int c = 0; c < ncomp; c++) {
     try {
       ok[c] = flow_pack_comp<T, C>(dom[c], dom[c + 1], rp, cj, val, upper, dinv, up_slot, lev.data(), pos.data(),
-                                   task_of.data(), part[c]);
+                                   task_of.data(), most_far, part[c]);
     } catch (const std::bad_alloc&) {
       ok[c] = 2;  // no exception may leave the parallel region
     }

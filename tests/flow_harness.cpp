@@ -396,6 +396,26 @@ int main() {
     make({0, 6000}, 0, 6000, 5000, 3, L2, U2, d2);
     if (solve<double, 1>(L2, U2, d2, {0, 6000}, 1, nullptr) != 2) bad++;
   }
+  // and factors of mostly far operands, where the caller sets a limit; far operands are no reason where they are few
+  {
+    using C = FlowCfg<float, 1>;
+    FlowPack<float> o;
+    auto pack = [&](int n, int deg, int back, long long most, int nsub) {
+      Tri L, U;
+      std::vector<double> dinv;
+      std::vector<int> dom = {0};
+      for (int c = 1; c <= nsub; c++) dom.push_back(n * c);
+      make(dom, deg, back, 0, 11, L, U, dinv);
+      auto uv = [&](int k) { return (float)U.va[k]; };
+      auto dv = [&](int i) { return (float)dinv[i]; };
+      return flow_pack<float, C>(n * nsub, U.rp.data(), U.cj.data(), uv, true, dom, &dv, nullptr, o, most);
+    };
+    if (!pack(50000, 6, 50000, LLONG_MAX, 1) || o.nfar < 75000) bad++;
+    const long long far = o.nfar;
+    if (pack(50000, 6, 50000, far / 2, 1) || !pack(50000, 6, 50000, 2 * far, 1)) bad++;
+    if (!pack(50000, 6, 50000, 2 * far, 2)) bad++;  // the limit is a subdomain's
+    if (!pack(50000, 6, 30, 0, 1)) bad++;
+  }
   std::printf("%d layouts solved, %d bad\n", packed, bad);
   return bad || packed < 100;
 }

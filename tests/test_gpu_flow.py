@@ -171,3 +171,40 @@ def test_factor_that_is_not_triangular_is_refused(bad):
                           lev_ptr=np.array([0, n], np.int32), levels=[lv], inner_enable=0)
     with pytest.raises(_abi.PgxError, match="triangular"):
         GemslrHandle(st, precision="fp64").close()
+
+
+def _many_far(n, deg):
+    """One subdomain, about `deg` entries a row anywhere before (after) it: levels of hundreds of rows."""
+    rng = np.random.default_rng(n)
+    out = []
+    for up in (False, True):
+        rows = np.repeat(np.arange(n, dtype=np.int64), deg)
+        cols = rng.integers(0, n, rows.size)
+        keep = cols > rows if up else cols < rows
+        key = np.unique(rows[keep] * n + cols[keep])
+        rp = np.concatenate([[0], np.cumsum(np.bincount(key // n, minlength=n))]).astype(np.int32)
+        out.append((rp, (key % n).astype(np.int32), rng.uniform(-1, 1, key.size) / deg, n, n))
+    return out[0], out[1], 1.0 + 0.2 * rng.uniform(-1, 1, n)
+
+
+@pytest.mark.parametrize("n,kernel", [(40000, "dataflow"), (90000, "segmented")])
+def test_factors_of_mostly_far_operands(n, kernel):
+    """On both sides of the number of far operands from which a subdomain leaves one SM; lanes follow their handle."""
+    from pargemslr_b200 import params as P
+    from pargemslr_b200.handle import GemslrHandle
+    L, U, dinv = _many_far(n, 40)
+    h = GemslrHandle(_one_level([0, n], L, U, dinv), precision="mixed")
+    try:
+        assert h.describe().count(kernel) >= 2  # the lower and the upper factor
+        B = np.random.default_rng(4).standard_normal((4, n))
+        ref = _substitute(L, U, dinv, B[0])
+        assert np.linalg.norm(h.apply(B[0]) - ref) <= 2e-5 * np.linalg.norm(ref)
+        p = P.workload_params("serve")
+        want = [h.solve(b, params=p)[0] for b in B]
+        h.set_lanes(4)
+        h.set_slots(2)
+        X, _ = h.solve_batch(B, params=p)
+        for k in range(4):
+            np.testing.assert_array_equal(X[k], want[k])
+    finally:
+        h.close()
