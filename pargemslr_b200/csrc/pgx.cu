@@ -3391,13 +3391,14 @@ struct Systems : SystemsBase {
     // chunk, first right-hand sides), a packed pass 0.7 us a level.  The
     // separators of these systems have one to three levels, their subdomains
     // hundreds.
-    t.nchunks = 0;
+    t.nchunks = t.wide = 0;
     if (t.nlev >= kSysFlowLevels) {
       FlowPack<P> pk;
       auto val = [&](int k) { return (P)h.va[k]; };
       auto diag = [&](int i) { return (P)(*dinv)[i]; };
       if (flow_pack<P, SysFlowCfg<P>>(nl, h.rp.data(), h.cj.data(), val, upper, {0, nl}, &diag, dst_map, pk)) {
         t.nchunks = (int)pk.chunk.size() / 4;
+        t.wide = pk.nfar > kSysMostFar && 2 * pk.nfar > h.nnz();
         ints(&t.chunk, pk.chunk.data(), pk.chunk.size());
         ints(&t.first, pk.first.data(), pk.first.size());
         const size_t at = images.size();

@@ -70,6 +70,7 @@ struct SysTri {
   // the same factor as task images (SysFlowCfg layout); no chunks: the
   // packed rows above are used
   int nchunks;
+  int wide;  // most operands of the images are far, and many: see kSysMostFar
   const int* chunk;
   const int* first;
   const unsigned char* blob;
@@ -358,6 +359,18 @@ __device__ __noinline__ void sys_trsv(const SysTri<P>& T, const P* rhs, P* out, 
   }
 }
 
+// A factor most of whose operands left the ring, and more than kSysMostFar of
+// them, is passed over by a large CTA's packed kernel in less time: seven
+// warps read those operands back from global memory, a packed pass has all of
+// the CTA's warps on a level.  16 systems of random matrices, 32 entries a row, in one launch
+// on a B200, dataflow / packed, ms:
+//                              256 threads             512 threads            1024 threads
+//   14,000 rows (154,000 far)   9.2/11.0, 11.4/14.0     7.6/8.5, 11.5/11.5     5.9/6.9, 8.3/9.0    (mixed, FP64)
+//   20,000 rows (245,000)      18.2/19.5, 23.6/25.8    15.9/15.5, 24.1/20.6   12.5/11.7, 17.3/15.3
+//   40,000 rows (560,000)      27.5/28.3, 33.3/33.2    23.0/18.4, 33.1/22.7   18.1/12.7, 23.9/15.0
+constexpr long long kSysMostFar = 200000;
+constexpr unsigned kSysWideThreads = 512;
+
 // One pass by dataflow (pgx_flow.cuh), the whole level as one subdomain.  The
 // chain of dependency levels bounds it, at about 0.15 us a level where the
 // barrier-a-level pass below takes 0.7: 40 systems of 32^2 to 112^2, mixed, in
@@ -394,7 +407,10 @@ __device__ void sys_solve_b(const SysDesc<P>& d, int l, const P* rhs, P* x, SysS
   const SysLevel<P>& v = d.lev[l];
   const unsigned ring = scap > 0 ? 1u << (31 - __clz(scap)) : 0u;
   const bool lr = v.L.span < (int)ring, ur = v.U.span < (int)ring;
-  if (sh.use_flow && v.L.nchunks > 0) {
+  auto by_flow = [&](const SysTri<P>& T) {
+    return sh.use_flow && T.nchunks > 0 && !(T.wide && blockDim.x >= kSysWideThreads);
+  };
+  if (by_flow(v.L)) {
     sys_flow<false, MAXT>(v.L, (const P*)d.yu, rhs, (P*)nullptr, sh);
   } else {
     constexpr int G = 4;  // gathers in flight per thread
@@ -415,7 +431,7 @@ __device__ void sys_solve_b(const SysDesc<P>& d, int l, const P* rhs, P* x, SysS
     else
       sys_trsv<false, 2, MAXT>(v.L, (const P*)d.yr, d.yu, lr ? sbuf : d.y, lr ? ring - 1 : 0xFFFFFFFFu);
   }
-  if (sh.use_flow && v.U.nchunks > 0)
+  if (by_flow(v.U))
     sys_flow<true, MAXT>(v.U, (const P*)d.yu, (const P*)nullptr, x, sh);
   else if (sh.depth == 3)
     sys_trsv<true, 3, MAXT>(v.U, (const P*)d.yu, x, ur ? sbuf : d.y, ur ? ring - 1 : 0xFFFFFFFFu);

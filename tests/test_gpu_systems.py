@@ -229,3 +229,22 @@ def test_packed_and_dataflow_passes_take_turns_in_one_buffer(precision):
     assert np.linalg.norm(first[0] - xs) <= 1e-6 * np.linalg.norm(xs)
     sb.close()
     h.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_systems_of_mostly_far_operands(precision):
+    """Random rows, whose passes a large CTA runs by its packed kernel and a small one by dataflow: both solve."""
+    from pargemslr_b200.handle import GemslrHandle
+    from pargemslr_b200.systems import SystemsBatch
+    p = P.workload_params("serve")
+    A = problems.random_diag_dominant(22000, 3)
+    h = GemslrHandle.from_matrix(A, p, precision=precision)
+    b = np.random.default_rng(2).standard_normal(22000)
+    systems = [(A, b, h)]
+    sb = SystemsBatch([h])
+    for sched in ((256, 2, 4, 2), (512, 1, 4, 2), (1024, 1, 4, 3)):
+        sb.set_schedule(*sched)
+        X, R = sb.solve([b], params=p)
+        _check_against_singles(systems, X, R, p)
+    sb.close()
+    h.close()
