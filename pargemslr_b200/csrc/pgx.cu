@@ -683,7 +683,14 @@ static bool want_segments(const HostCsr& h, int nnz_cap) {
 // instead of two passes: ncu on a B200, 64^3 mixed, 6 us for the product, 19
 // us for each pass, 25 B-solves of this kind a preconditioner call.  Entries
 // are formed in FP64 and rounded once.
+// No entry of M may exceed kDirectGrowth times the largest |D_ii|: a product
+// that forms large entries to cancel them rounds more than the passes do, and
+// its entries may leave the range of a float where no result of a pass does.
+// In a CPU model of eight levels in FP32 (b = A x), its error is 0.8 to 1.2 of
+// the passes' with multipliers up to 1 and 2.4 to 3.4 times it from 3 on.  198 products of
+// this library's setups had no entry above 1.04 times the largest |D_ii|.
 constexpr int kDirectLevels = 8;
+constexpr double kDirectGrowth = 4.0;
 template <typename S>
 static bool shallow_inverse(const HostCsr& L, const HostCsr& U, const std::vector<double>& dinv, HostCsr& M) {
   const int n = L.rows;
@@ -697,6 +704,10 @@ static bool shallow_inverse(const HostCsr& L, const HostCsr& U, const std::vecto
       if (lev[i] >= kDirectLevels) return false;
     }
   }
+  double dmax = 0.0;
+  for (int i = 0; i < n; i++) dmax = std::max(dmax, (double)std::abs(((const S*)dinv.data())[i]));
+  const double top = kDirectGrowth * dmax;
+  if (!std::isfinite(top)) return false;
   const size_t limit = 2 * ((size_t)n + (size_t)L.nnz() + (size_t)U.nnz());
   const S *lv = (const S*)L.va.data(), *uv = (const S*)U.va.data(), *dv = (const S*)dinv.data();
   // rows of an inverse, formed in solving order: row_i = d_i (e_i - sum_j T_ij row_j)
@@ -749,6 +760,7 @@ static bool shallow_inverse(const HostCsr& L, const HostCsr& U, const std::vecto
     row.clear();
     if (!take(row, count)) return false;
     for (const auto& e : row) {
+      if (!(std::abs(e.second) <= top)) return false;
       M.cj.push_back(e.first);
       const double* v = (const double*)&e.second;
       M.va.insert(M.va.end(), v, v + vw);

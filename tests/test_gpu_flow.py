@@ -156,6 +156,44 @@ def test_shallow_factors(levels, cplx):
     assert np.linalg.norm(z - ref) <= 1e-14 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("size", [0.5, 300.0, 1e12])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_shallow_factors_that_grow_keep_their_passes(size, precision):
+    """Five levels of large multipliers: the product of the inverses would hold entries of size^4 times those of D^-1
+    (at 1e12 beyond a float's range), and results that need none of them would be lost."""
+    from pargemslr_b200.handle import GemslrHandle
+    n, step = 1000, 200  # five rows a chain
+    rows = np.arange(step, n)
+    rp = np.concatenate([np.zeros(step, np.int32), np.arange(n - step + 1, dtype=np.int32)])
+    up = np.concatenate([np.arange(n - step + 1, dtype=np.int32), np.full(step, n - step, np.int32)])
+    rng = np.random.default_rng(7)
+    L = (rp, (rows - step).astype(np.int32), size * rng.uniform(0.5, 1, n - step), n, n)
+    U = (up, rows.astype(np.int32), size * rng.uniform(0.5, 1, n - step), n, n)
+    dinv = 1.0 + rng.random(n)
+    b = rng.standard_normal(n)
+    b[:600] = 0.0  # what is left reaches two levels on
+    b[600:] *= 1e-9 if size > 1e6 else 1.0
+    h = GemslrHandle(_one_level([0, n], L, U, dinv), precision=precision)
+    try:
+        assert ("product of the inverses" in h.describe()) == (size < 1)
+        z = h.apply(b)
+    finally:
+        h.close()
+    kind = np.float64 if precision == "fp64" else np.float32
+    y = b.astype(kind)
+    for i in range(step, n):
+        y[i] -= kind(L[2][i - step]) * y[i - step]
+    y *= dinv.astype(kind)
+    for i in range(n - step - 1, -1, -1):
+        y[i] -= kind(dinv[i]) * kind(U[2][i]) * y[i + step]
+    fin = np.isfinite(y)
+    assert fin[600:].all()
+    # two steps each way, a few roundings each, in either order
+    tol = 1e-14 if precision == "fp64" else 5e-6
+    for a in (600, 800):
+        assert np.linalg.norm(z[a:a + step] - y[a:a + step]) <= tol * np.linalg.norm(y[a:a + step].astype(np.float64))
+
+
 @pytest.mark.parametrize("bad", ["L", "U"])
 def test_factor_that_is_not_triangular_is_refused(bad):
     from pargemslr_b200 import _abi
