@@ -307,6 +307,17 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
       for (int u = 0; u < 4; u++)
 #pragma unroll
         for (int r = 0; r < R; r++) acc[e][u][r] = T(0);
+    T old[R];  // the sum of all but the last quad; one set of sums: of the blocks that are complete
+#pragma unroll
+    for (int r = 0; r < R; r++) old[r] = T(0);
+    auto fold = [&]() {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        old[r] += (acc[0][0][r] + acc[0][2][r]) + (acc[0][1][r] + acc[0][3][r]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) acc[0][u][r] = T(0);
+      }
+    };
     // far operands: solved so long ago that they left the ring.  Their tasks
     // are 3 W back: this warp's last wait covers the release after their stores.
     constexpr int FQ = R == 1 ? 2 : 1;  // far quads whose loads are in flight together
@@ -333,7 +344,13 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
         }
       }
 #pragma unroll
-      for (int e = 0; e < FQ; e++)
+      for (int e = 0; e < FQ; e++) {
+        if constexpr (kFlowSets<T> == 1) {
+          bool next = false;
+#pragma unroll
+          for (int u = 0; u < 4; u++) next |= cc[e][u] >= 0 && (cc[e][u] & kFlowOther);
+          if (next) fold();
+        }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
           const bool newest = (cc[e][u] & kFlowLast) != 0;
@@ -350,6 +367,7 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
               acc[0][u][r] = t;
           }
         }
+      }
     }
     flow_wait<C::W>(s_prog, h1.y, lane, err, &s_abort);
     // the slots of the rows half a ring ahead: their old values are read no more
@@ -365,7 +383,13 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     int k = 0;
     FlowQuad<T> cur;
     if (g4 > 0) cur = flow_load_quad<T>(cols, vals, l);
+    // before the oldest quad of a block, unless the far operands began it (or the row has nothing in it)
+    auto next_block = [&]() {
+      if constexpr (kFlowSets<T> == 1)
+        if ((g4 - k) % kFlowBlock == 0 && (cur.c.x & 0xffffu) != (unsigned)C::ring) fold();
+    };
     auto use = [&](T (&s)[4][R]) {
+      next_block();
       FlowQuad<T> nxt = cur;
       if (k + 1 < g4) nxt = flow_load_quad<T>(cols, vals, (k + 1) * stride + l);
       const unsigned i0 = cur.c.x & 0xffffu, i1 = cur.c.x >> 16, i2 = cur.c.y & 0xffffu, i3 = cur.c.y >> 16;
@@ -433,6 +457,7 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
       }
     };
     auto fresh = [&](T (&s)[4][R]) {
+      next_block();
       const FlowQuad<T> nxt = flow_load_quad<T>(cols, vals, (k + 1) * stride + l);
       poll(cur);
 #pragma unroll
@@ -449,14 +474,14 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
       fresh(acc[0]);
       if (kFlowSets<T> == 2 && k + 1 < g4) fresh(acc[kFlowSets<T> - 1]);
     }
-    // the sum of all but the last quad, formed before that is waited for
-    T old[R];
+    // the sum of all but the last quad is formed before that is waited for
 #pragma unroll
     for (int r = 0; r < R; r++) {
       T part[4];
 #pragma unroll
       for (int u = 0; u < 4; u++) part[u] = kFlowSets<T> == 2 ? acc[0][u][r] + acc[kFlowSets<T> - 1][u][r] : acc[0][u][r];
-      old[r] = (part[0] + part[2]) + (part[1] + part[3]);
+      const T sum = (part[0] + part[2]) + (part[1] + part[3]);
+      old[r] = kFlowSets<T> == 2 ? sum : old[r] + sum;
     }
     if (g4 > 0) {
       poll(cur);

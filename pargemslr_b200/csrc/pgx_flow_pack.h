@@ -14,16 +14,26 @@ namespace pgx {
 
 constexpr int kFlowHead = 16;                  // ints of a task header
 constexpr int kFlowMaxQuads = 250;             // quads of one row (a byte each in the header)
-constexpr int kFlowOther = 1 << 30;            // far operand: the set of accumulators the second quad uses
+constexpr int kFlowOther = 1 << 30;            // far operand: the second set of sums; with one set, see kFlowBlock
 constexpr int kFlowLast = 1 << 29;             // far operand: one of the row's four newest entries
 constexpr int kFlowIndex = kFlowLast - 1;
 // A row's four newest entries are summed by themselves, the others in
 // kFlowSets sets of four accumulators, successive quads on alternate sets: as
-// many partial sums as the eight lanes a row that summed it before, and no
-// more rounding (the lower pass at 48^3 in FP32 against
-// FP64: 4.1e-8 with eight, 4.4e-8 with four, 4.9e-8 with two).
+// many partial sums as the eight lanes that summed a row before (sixteen where
+// a factor has more than 32 entries a row), and no more rounding up to that length (the
+// lower pass at 48^3 in FP32 against FP64: 4.1e-8 with eight, 4.4e-8 with
+// four, 4.9e-8 with two; in a CPU model of 67 / 201 entries a row sixteen sums
+// round 0 to 8% / 12 to 17% less than eight).
 template <typename T>
 constexpr int kFlowSets = sizeof(T) <= 8 ? 2 : 1;
+// Two sets of 16-byte values do not fit the registers (four lanes spilled, and
+// took twice the time).  There the one set is added up after every kFlowBlock
+// quads, counted from the row's end, and starts again from zero.  Error of a
+// pass against 80 bits in a CPU model (ILUT factors of shifted 3D Laplacians),
+// as a multiple of eight lanes' error, 35 / 67 / 201 entries a row: 1.00 to
+// 1.02 / 0.96 to 0.97 / 0.94; with the set running through 1.03 to 1.05 /
+// 1.08 / 1.23 to 1.24.
+constexpr int kFlowBlock = 8;
 
 // Whether a warp may test the barrier of chunk `chunk`, with `issued` chunks
 // issued so far.  Chunk c uses the stage and the barrier of chunk c - stages
@@ -258,7 +268,7 @@ static bool flow_pack_comp(int r0, int r1, const int* rp, const int* cj, const V
           *cp = upper ? cj[k] : (*up_slot)[cj[k]];
           if (back < 4)
             *cp |= kFlowLast;
-          else if (kFlowSets<T> == 2 && (back / 4 + quads + 1) % 2)
+          else if (kFlowSets<T> == 2 ? (back / 4 + quads + 1) % 2 : back / 4 % kFlowBlock == kFlowBlock - 1)
             *cp |= kFlowOther;
           *vp = val(k);
         } else {
