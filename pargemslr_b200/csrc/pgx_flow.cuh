@@ -55,22 +55,22 @@ __device__ __forceinline__ void flow_add(unsigned* p) {
   asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(p)) : "memory");
 }
 // until every task below `lim` is done (bounded); task t belongs to warp t % W, prog[w] counts warp w's done tasks.
-// A warp gives up as a whole: its lanes meet in votes and warp barriers again.
+// A warp gives up as a whole: its lanes meet in votes and warp barriers again.  Returns prog[W] (0 if it gave up).
 template <int W>
-__device__ __forceinline__ void flow_wait(unsigned* prog, int lim, int lane, int* err, unsigned* abort) {
+__device__ __forceinline__ unsigned flow_wait(unsigned* prog, int lim, int lane, int* err, unsigned* abort) {
   const unsigned need = lane < W && lim > lane ? (unsigned)(lim - lane + W - 1) / W : 0u;
   for (int k = 0;; k++) {
-    const unsigned v = lane < W ? flow_ld(&prog[lane]) : 0u;
+    const unsigned v = lane <= W ? flow_ld(&prog[lane]) : 0u;
     if (__all_sync(0xffffffffu, v >= need)) {
       __syncwarp();  // a vote orders no memory: the lanes that acquired hand over to the others here
-      return;
+      return __shfl_sync(0xffffffffu, v, W);
     }
     if ((k & 255) == 255) {
       if (k >= kFlowPolls) {
         atomicOr(err, kErrStage);
         *(volatile unsigned*)abort = 1u;
       }
-      if (__any_sync(0xffffffffu, *(volatile unsigned*)abort != 0)) return;
+      if (__any_sync(0xffffffffu, *(volatile unsigned*)abort != 0)) return 0u;
     }
   }
 }
@@ -179,9 +179,37 @@ __device__ __forceinline__ FlowQuad<T> flow_load_quad(const unsigned char* cols,
 template <typename C>
 struct FlowShared {
   unsigned long long full[C::stages];  // a chunk has landed
-  unsigned prog[C::W], freed[C::stages], abort;
-  unsigned issued;  // chunks whose copies are issued
+  unsigned prog[C::W + 1];  // tasks each warp has done; chunks whose copies are issued
+  unsigned freed[C::stages], abort;
 };
+
+// Until chunk `ch` has landed (bounded); `issued`: the number of chunks that
+// the warp knows to be issued.  The abort flag is looked at only where a wait
+// does not end at once, and the count of issued chunks comes with the progress
+// (flow_wait): both lie between a warp's tasks, which wait for little else
+// where rows are short.  With a look at each once a task, B200: a 61x55x64
+// imported application (FP64) 544 us, now 509; 256^2 FP64 solve 98.5 and 95.0
+// ms; 64^3 mixed 84.0 and 82.9 ms.  Returns false, to every lane, when a wait gave up.
+template <typename C>
+__device__ __forceinline__ bool flow_chunk(FlowShared<C>& sh, int ch, unsigned& issued, int* err) {
+  unsigned long long* const bar = &sh.full[ch % C::stages];
+  const unsigned parity = (unsigned)((ch / C::stages) & 1);
+  if (flow_issued(issued, ch) && __all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  for (;;) {
+    if (!flow_issued(issued, ch)) {
+      if (__all_sync(0xffffffffu, flow_issued(flow_ld(&sh.prog[C::W]), ch))) issued = (unsigned)ch + 1u;
+    } else if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+      return true;
+    }
+    const bool late = clock64() - t0 >= kMbarWaitCycles;
+    if (late) atomicOr(err, kErrStage);
+    if (__any_sync(0xffffffffu, late || *(volatile unsigned*)&sh.abort != 0)) {
+      *(volatile unsigned*)&sh.abort = 1u;
+      return false;
+    }
+  }
+}
 
 // One pass over subdomain `comp`, whose chunks are a.chunk[c0 .. c0 + nch):
 // called by every thread of a CTA of at least C::threads threads; the caller
@@ -206,10 +234,9 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
       mbar_init(&s_full[s], 1);
       s_freed[s] = 0;
     }
-    sh.issued = 0;
     mbar_fence_init();
   }
-  if (tid < C::W) s_prog[tid] = 0;
+  if (tid <= C::W) s_prog[tid] = 0;
   {
     unsigned* w = (unsigned*)smem_raw;
     constexpr int words = C::ring * (int)sizeof(V) / 4;
@@ -254,7 +281,7 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
               mbar_arrive_expect_tx(&s_full[s], (unsigned)m.y * 16u);
               bulk_g2s(stage0 + (size_t)s * C::stage_bytes, a.blob + (size_t)m.x * 16, (unsigned)m.y * 16u, &s_full[s]);
               c++;
-              flow_st(&sh.issued, (unsigned)c);
+              flow_st(&s_prog[C::W], (unsigned)c);
             }
           }
         }
@@ -272,21 +299,10 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
   for (int r = 0; r < R; r++) b[r] = T(0);
   const unsigned ring_at = smem_u32(smem_raw);
   unsigned mine = 0;    // tasks this warp has done
-  unsigned issued = 0;  // chunks this lane knows to be issued
+  unsigned issued = 0;  // chunks this warp knows to be issued
   while (ch >= 0) {
-    for (int k = 0; !flow_issued(issued, ch) && !*(volatile unsigned*)&s_abort; k++) {
-      issued = flow_ld(&sh.issued);
-      if (k >= kFlowPolls) {
-        atomicOr(err, kErrStage);
-        *(volatile unsigned*)&s_abort = 1u;
-      }
-    }
-    if (__any_sync(0xffffffffu, *(volatile unsigned*)&s_abort != 0)) break;
     const int st = ch % D;
-    if (!__all_sync(0xffffffffu, mbar_wait(&s_full[st], (unsigned)((ch / D) & 1), err))) {
-      s_abort = 1;
-      break;
-    }
+    if (!flow_chunk<C>(sh, ch, issued, err)) break;
     const unsigned char* base = stage0 + (size_t)st * C::stage_bytes;
     const int4 h0 = *(const int4*)(base + off), h1 = *(const int4*)(base + off + 16),
                h2 = *(const int4*)(base + off + 32), h3 = *(const int4*)(base + off + 48);
@@ -369,7 +385,8 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
         }
       }
     }
-    flow_wait<C::W>(s_prog, h1.y, lane, err, &s_abort);
+    // with the progress comes the number of chunks issued, in time for the look ahead at the end of the task
+    issued = max(issued, flow_wait<C::W>(s_prog, h1.y, lane, err, &s_abort));
     // the slots of the rows half a ring ahead: their old values are read no more
     if (on) {
       FlowVal<T, R> none;
@@ -427,7 +444,7 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     };
     run(min(g1, g4 - 1));
     if (g2 > g1) {
-      flow_wait<C::W>(s_prog, h1.z, lane, err, &s_abort);
+      issued = max(issued, flow_wait<C::W>(s_prog, h1.z, lane, err, &s_abort));
       run(min(g2, g4 - 1));
     }
     // what the end of the task needs, and the right-hand side of this warp's next task
@@ -518,7 +535,6 @@ __device__ __forceinline__ void flow_pass(FlowShared<C>& sh, unsigned char* smem
     T bn[R];
 #pragma unroll
     for (int r = 0; r < R; r++) bn[r] = T(0);
-    if (nch_ >= 0 && !flow_issued(issued, nch_)) issued = flow_ld(&sh.issued);
     if (nch_ >= 0 && flow_issued(issued, nch_) && mbar_try_wait(&s_full[nch_ % D], (unsigned)((nch_ / D) & 1))) {
       const unsigned char* nbase = stage0 + (size_t)(nch_ % D) * C::stage_bytes;
       const int nr2 = *(const int*)(nbase + noff + 12) & 0xff;
