@@ -246,3 +246,41 @@ def test_factors_of_mostly_far_operands(n, kernel):
             np.testing.assert_array_equal(X[k], want[k])
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+@pytest.mark.parametrize("name", ["two narrow subdomains and an empty one", "long rows", "operands older than the ring"])
+def test_infinities_and_nan_pass_through(name, cplx, precision):
+    """A result that is not finite is a result: rows that depend on it are not finite either, in class as plain
+    substitution has them (real values), and all others are as without it."""
+    from pargemslr_b200.handle import GemslrHandle
+    dom, deg, back, longrow = CASES[name]
+    L, U, dinv = _factors(dom, deg, back, len(name), cplx, longrow)
+    n = dom[-1]
+    h = GemslrHandle(_one_level(dom, L, U, dinv), precision=precision)
+    try:
+        assert "dataflow" in h.describe()
+        b = np.random.default_rng(3).standard_normal(n) + (1j if cplx else 0.0)
+        import torch
+        for bad in (np.inf, -np.inf, np.nan):
+            for at in (n - 2, n // 2):  # reaches few rows, and many
+                v = b.copy()
+                v[at] = bad
+                with np.errstate(all="ignore"):
+                    ref = _substitute(L, U, dinv, v)
+                vd = torch.from_numpy(v).cuda()
+                zd = torch.zeros_like(vd)
+                from pargemslr_b200 import _abi
+                _abi.check(_abi.lib().pgx_gemslr_precond_apply(h._h, zd.data_ptr(), vd.data_ptr(), _abi.LOCATION_DEVICE))
+                z = zd.cpu().numpy()
+                fin = np.isfinite(ref)
+                assert fin.any() and not fin.all()
+                np.testing.assert_array_equal(np.isfinite(z), fin)
+                if not cplx:
+                    np.testing.assert_array_equal(np.isnan(z), np.isnan(ref))
+                    np.testing.assert_array_equal(np.sign(z[np.isinf(z)]), np.sign(ref[np.isinf(ref)]))
+                tol = 1e-13 if precision == "fp64" else 2e-5
+                assert np.linalg.norm(z[fin] - ref[fin]) <= tol * np.linalg.norm(ref[fin])
+    finally:
+        h.close()
