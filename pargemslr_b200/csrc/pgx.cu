@@ -3985,7 +3985,7 @@ int pgx_gemslr_commit(pgx_handle h) {
   h->extra.clear();
   h->eng.reset();
   // laying out the factors allocates host memory: no exception may cross the C ABI
-  return guarded("pgx_gemslr_commit", [&]() -> int {
+  const int rc = guarded("pgx_gemslr_commit", [&]() -> int {
     switch (im.precision) {
       case PGX_PRECISION_MIXED: {
         auto* e = new Engine<float>();
@@ -4013,6 +4013,8 @@ int pgx_gemslr_commit(pgx_handle h) {
     }
     return PGX_SUCCESS;
   });
+  if (rc != PGX_SUCCESS) h->eng.reset();  // half an engine must not be solved with
+  return rc;
 }
 
 // ------------------------------------------------------------ host setup

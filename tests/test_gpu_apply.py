@@ -69,3 +69,42 @@ def test_applications_without_device_memory_left():
         keep.clear()
         torch.cuda.empty_cache()
         h.close()
+
+
+def test_a_failed_commit_leaves_nothing_to_solve_with():
+    """A handle whose commit was refused answers as one that was never committed, and can be committed again."""
+    from pargemslr_b200.handle import import_structures, init
+    from pargemslr_b200.structures import GemslrStructures, LevelStructures, empty_csr
+    init(0)
+    n = 40
+    eye = (np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32), np.ones(n), n, n)
+    rp = np.zeros(n + 1, np.int32)
+    rp[8:] = 1  # one entry, in row 7, on the wrong side of the diagonal
+    bad = (rp, np.array([9], np.int32), np.ones(1), n, n)
+
+    def structures(L):
+        lv = LevelStructures(ncomp=1, dom_ptr=np.array([0, n], np.int32), L=L, U=empty_csr(n, n), dinv=np.ones(n), B=eye)
+        return GemslrStructures(n=n, A=eye, pperm=np.arange(n, dtype=np.int32), qperm=None,
+                                lev_ptr=np.array([0, n], np.int32), levels=[lv], inner_enable=0)
+
+    lib = _abi.lib()
+    h = import_structures(structures(bad), "fp64")
+    try:
+        assert lib.pgx_gemslr_commit(h) != 0
+        v, z = np.ones(n), np.zeros(n)
+        assert lib.pgx_gemslr_precond_apply(h, _abi.ptr(z), _abi.ptr(v), _abi.LOCATION_HOST) != 0
+        assert b"before commit" in lib.pgx_last_error()
+        keep = []
+        desc = _abi.Level()
+        lv = structures(empty_csr(n, n)).levels[0]
+        keep += [np.ascontiguousarray(lv.dom_ptr, np.int32), _abi.doubles(lv.dinv)]
+        desc.ncomp, desc.dom_ptr, desc.dinv = 1, _abi.ptr(keep[0]), _abi.ptr(keep[1])
+        for name in ("L", "U", "B"):
+            setattr(desc, name, _abi.csr_struct(*getattr(lv, name), keep=keep))
+        import ctypes as C
+        _abi.check(lib.pgx_gemslr_set_level(h, 0, C.byref(desc)))
+        _abi.check(lib.pgx_gemslr_commit(h))
+        _abi.check(lib.pgx_gemslr_precond_apply(h, _abi.ptr(z), _abi.ptr(v), _abi.LOCATION_HOST))
+        np.testing.assert_array_equal(z, v)
+    finally:
+        lib.pgx_gemslr_destroy(h)
