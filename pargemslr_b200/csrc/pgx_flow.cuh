@@ -18,14 +18,14 @@
 //   - results sit in a shared-memory ring by schedule position.  A slot not
 //     solved yet holds a signalling NaN, so a consumer polls the value itself:
 //     one store and one load a level.  (A progress counter beside the value
-//     took 270 ns a level where this takes 140, with or without its fences;
-//     a CTA barrier a level took 600-900.)
+//     took 270 ns a level where this takes 130 to 160, with or without its
+//     fences; a CTA barrier a level took 600-900.)
 //   - one more warp streams the factor into shared memory by bulk copies.
 // On a B200, level 0 of the 7-point Laplacian at 64^3 (ILUT 1e-3), lower /
-// upper pass: 0.29 / 0.28 ms mixed and 0.46 / 0.43 ms FP64, one lane (one
-// barrier a level: 1.30 / 1.19 and 1.64 / 1.52 ms); 0.47 / 0.45 ms for four
-// lanes mixed.  At 128^3, mixed: 2.0 / 1.8 ms one lane (6.04 / 5.76), 4.6 /
-// 4.0 ms four lanes.
+// upper pass: 0.32 / 0.30 ms mixed and 0.50 / 0.47 ms FP64, one lane (one
+// barrier a level: 1.30 / 1.19 and 1.64 / 1.52 ms); 0.51 / 0.46 ms for four
+// lanes mixed.  At 128^3, mixed: 2.1 / 1.9 ms one lane (6.04 / 5.76), 4.7 /
+// 4.1 ms four lanes.
 #pragma once
 
 #include "pgx_device.cuh"
