@@ -184,8 +184,9 @@ def test_shallow_factors_that_grow_keep_their_passes(size, precision):
     for i in range(step, n):
         y[i] -= kind(L[2][i - step]) * y[i - step]
     y *= dinv.astype(kind)
-    for i in range(n - step - 1, -1, -1):
-        y[i] -= kind(dinv[i]) * kind(U[2][i]) * y[i + step]
+    with np.errstate(over="ignore"):  # the rows that leave a float's range are not looked at
+        for i in range(n - step - 1, -1, -1):
+            y[i] -= kind(dinv[i]) * kind(U[2][i]) * y[i + step]
     fin = np.isfinite(y)
     assert fin[600:].all()
     # two steps each way, a few roundings each, in either order
